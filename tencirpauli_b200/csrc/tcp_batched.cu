@@ -317,7 +317,7 @@ int configure_ring(tcp_mvp_batch *b) {
         const tcp_mvp_plan *p = b->plans[h];
         b->hams_host[h].dim = p->dim;
         b->hams_host[h].nqubits = p->nqubits;
-        if (p->sched.dev.ring_steps == 0) {
+        if (p->sched.dev.ring[0].steps == 0) {
             b->empty_members.push_back(static_cast<uint32_t>(h));
             continue;
         }

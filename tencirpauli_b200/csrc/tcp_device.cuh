@@ -28,6 +28,17 @@ constexpr uint32_t kNoPasses = 0xffffffffu;
 constexpr int kErrTimeout = 1;
 constexpr int kErrBounds = 2;  // TCP_DEBUG_BOUNDS builds: a block failed its bounds check
 
+// Ring view (k_ring; see tcp::RingSchedule): steps = 0 when the plan has no
+// schedule of this shape.  Pass ranges as in DevSchedule, over the ring steps.
+struct RingView {
+    const uint4 *info;              // 4 words per step, see tcp::RingSchedule::step_info
+    const unsigned char *blocks128;  // blocks with FP64 weights
+    const unsigned char *blocks64;   // blocks with FP32 weights
+    uint32_t steps;
+    uint32_t pass_begin[kPassChunks + 1];
+    uint32_t pass_shift;
+};
+
 struct DevSchedule {
     // step view (tiled kernels); see tcp::Schedule
     const uint4 *step_info;          // d lo, d hi, block offset / 16, ngroups | (bytes / 16) << 16
@@ -43,14 +54,7 @@ struct DevSchedule {
     // than kPassChunks tiles.
     uint32_t pass_begin[kPassChunks + 1];
     uint32_t pass_shift;
-    // ring view (k_ring; see tcp::RingSchedule): ring_steps = 0 when the
-    // plan has no ring schedule.  Pass ranges as above, over the ring steps.
-    const uint4 *ring_info;          // d lo, d hi, block offset / 16, block bytes / 16
-    const unsigned char *ring128;    // blocks with FP64 weights
-    const unsigned char *ring64;     // blocks with FP32 weights
-    uint32_t ring_steps;
-    uint32_t ring_pass_begin[kPassChunks + 1];
-    uint32_t ring_pass_shift;
+    RingView ring[tcp::kRingShapeCount];  // k_ring's schedules, one per shape
     // group view (row kernel, transition count, diagonal): unfolded weights
     const uint64_t *g_mask;
     const uint32_t *g_tbeg;
@@ -159,6 +163,44 @@ __device__ __forceinline__ bool mbar_wait_or_abort(uint64_t *bar, uint32_t parit
     }
 }
 
+// ------------------------------ tensor memory ------------------------------
+// Tensor memory as a register extension: a warp reads and writes its own 32
+// lanes (warp % 4), one 32-bit word per lane and column.
+__device__ __forceinline__ void tmem_alloc(uint32_t *smem_addr, uint32_t columns) {
+    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;\n"
+                 "tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::"r"(smem_u32(smem_addr)), "r"(columns)
+                 : "memory");
+}
+__device__ __forceinline__ void tmem_dealloc(uint32_t addr, uint32_t columns) {
+    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(addr), "r"(columns) : "memory");
+}
+// 16 words of the lane: 8 64-bit values, low words first.
+__device__ __forceinline__ void tmem_load8(uint32_t addr, uint64_t (&v)[8]) {
+    uint32_t w[16];
+    asm volatile(
+        "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15}, [%16];\n"
+        "tcgen05.wait::ld.sync.aligned;"
+        : "=r"(w[0]), "=r"(w[1]), "=r"(w[2]), "=r"(w[3]), "=r"(w[4]), "=r"(w[5]), "=r"(w[6]), "=r"(w[7]), "=r"(w[8]),
+          "=r"(w[9]), "=r"(w[10]), "=r"(w[11]), "=r"(w[12]), "=r"(w[13]), "=r"(w[14]), "=r"(w[15])
+        : "r"(addr)
+        : "memory");
+#pragma unroll
+    for (int k = 0; k < 8; ++k) asm("mov.b64 %0, {%1, %2};" : "=l"(v[k]) : "r"(w[2 * k]), "r"(w[2 * k + 1]));
+}
+__device__ __forceinline__ void tmem_store8(uint32_t addr, const uint64_t (&v)[8]) {
+    uint32_t w[16];
+#pragma unroll
+    for (int k = 0; k < 8; ++k) asm("mov.b64 {%0, %1}, %2;" : "=r"(w[2 * k]), "=r"(w[2 * k + 1]) : "l"(v[k]));
+    asm volatile(
+        "tcgen05.st.sync.aligned.32x32b.x16.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, %16};" ::"r"(
+            addr),
+        "r"(w[0]), "r"(w[1]), "r"(w[2]), "r"(w[3]), "r"(w[4]), "r"(w[5]), "r"(w[6]), "r"(w[7]), "r"(w[8]), "r"(w[9]),
+        "r"(w[10]), "r"(w[11]), "r"(w[12]), "r"(w[13]), "r"(w[14]), "r"(w[15])
+        : "memory");
+}
+// The warp's stores have reached tensor memory.
+__device__ __forceinline__ void tmem_wait_stores() { asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory"); }
+
 // ------------------------------ complex types ------------------------------
 template <typename R> struct Cx;
 template <> struct Cx<double> { using T = double2; };
@@ -266,7 +308,8 @@ template <> struct Acc<float> {
 // the scalar instruction), so one instruction serves both components.  Two
 // running partial sums -- p for real weights (w x) and q for imaginary
 // weights (w x, whose contribution is i q) -- take the same instruction form;
-// compensate() folds p + i q into the Kahan-compensated row sum.
+// fold() adds p + i q to the Kahan-compensated row sum, which the kernel keeps
+// in registers (8 rows per thread) or in tensor memory (16 rows).
 template <typename R> struct RingAcc;
 template <> struct RingAcc<double> : Acc<double> {};
 
@@ -297,11 +340,11 @@ __device__ __forceinline__ uint64_t sub2(uint64_t a, uint64_t b) {
 }
 
 template <> struct RingAcc<float> {
-    uint64_t s = 0, c = 0;  // Kahan sum and compensation, (re, im)
     uint64_t p = 0, q = 0;  // running partial sums of real / imaginary weights
     __device__ __forceinline__ void add_real(float w, float2 v) { p = fma2(pack2(w, w), pack2(v.x, v.y), p); }
     __device__ __forceinline__ void add_imag(float w, float2 v) { q = fma2(pack2(w, w), pack2(v.x, v.y), q); }
-    __device__ __forceinline__ void compensate() {
+    // Fold p + i q into the Kahan sum s with compensation c, both (re, im).
+    __device__ __forceinline__ void fold(uint64_t &s, uint64_t &c) {
         const float2 qq = unpack2(q);
         const uint64_t term = add2(p, pack2(-qq.y, qq.x));  // p + i q
         const uint64_t yv = sub2(term, c);
@@ -310,7 +353,6 @@ template <> struct RingAcc<float> {
         s = tv;
         p = q = 0;
     }
-    __device__ __forceinline__ float2 value() const { return unpack2(s); }
 };
 
 }  // namespace tcpdev

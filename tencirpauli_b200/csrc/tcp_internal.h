@@ -95,35 +95,83 @@ struct Schedule {
 // so the values are loaded once per coset, in row order (fixed offsets), and
 // every group of the coset applies them through a compile-time register
 // permutation a = jh (its inner-mask bits above the thread bits).
-// Block layout (16-byte units):
-//   header    {ncosets, ngroups, terms offset / 16, 0}
-//   cosets    {m_lo, 0, groups in the coset, 0} each
-//   groups    u32 each: a | nterms << 4, padded to 16 bytes; a group's
-//             records come in four runs (real weights with one sign for all
-//             rows of a thread, real with a row pattern, then the same for
-//             imaginary weights)
-//   terms     16 bytes each: meta = zlo | pattern << 9 | imag << 17, zt32 =
-//             z >> S (low 32 bits), then the folded weight: one f64
-//             (complex128 blocks) or one f32 + 4 pad bytes (complex64 blocks).
-// A weight is real (imag = 0) or imaginary (imag = 1); a term with a complex
-// weight is stored as two records with the same z.  The folded sign is
-// parity(zt & d) ^ parity(zlo & m_lo) ^ parity(zj & jh) as in Schedule, so the
-// remaining sign of row j is parity(zlo & t) ^ parity(zt & tile) ^ bit j of
-// the pattern.  Needs n - S <= 32 (zt32 holds every outer z bit).
+//
+// A group's terms are cut into runs: one run per kind of weight (real or
+// imaginary) and per row part zj of the z mask (its bits above the thread
+// bits).  Inside a run the signs of a thread's 8 source values differ only by
+// parity(zj & s) of the source row s, the same for every thread, so the kernel
+// keeps the loaded values multiplied by that sign (a run names the bits in
+// which its zj differs from the run before), sums the run's signed weights
+// into one scalar D per thread and multiplies the 8 values by it: the work per
+// term is a sign and an addition per thread, the multiply-adds are paid once
+// per run.
+// The sign of a term is parity(zs & c) with zs = zlo | zt << 9 against the
+// thread's constant word c = t | tile << 9 (hence n - 3 <= 32); parity(zt & d)
+// ^ parity(zlo & m_lo) is folded into the weight.
+//
+// The signed sum of a run takes two forms, mixed freely:
+//   singles   one record per term: zs and weight;
+//   tables    terms whose zs lie in one affine space z0 ^ span(v1 .. vr),
+//             r <= 4: their sum is (-1)^parity(z0 & c) T[i] with bit k of i =
+//             parity(v_{k+1} & c) and T the 2^r signed sums of the weights,
+//             formed in double precision when the plan is built.
+// A table costs about as much as 2 to 4 singles whatever the number of its
+// terms: Jordan-Wigner two-body groups (16 terms in a 4-dimensional space)
+// take one table of 16.
+//
+// A step's block is one stream of records, walked front to back:
+//   header    {record count, 0, 0, 0}
+//   record    {zs or z0, word, ...}: single {.., f64 weight} or (complex64)
+//             {.., f32 weight, 0}; table of 4 {.., v1, v2} and 4 weights; table
+//             of 8 or 16 {.., v1, v2}, {v3, v4 or 0, 0, 0} and the weights
+// The word (kRing* below) names the run (a, imag, row signs to flip) and tells
+// where it ends, where a coset begins (the 8 source values are loaded then)
+// and, complex64, where the partial sums are folded into the compensated row
+// sums (a new coset follows a fold, so no loaded values live across it).  Records are 16-byte aligned and the next one is loaded while the
+// present one is applied, so a block leaves 16 bytes of its stage unused.
+constexpr uint32_t kRingImag = 1u << 4;       // bits 0..3: the register permutation a
+constexpr uint32_t kRingKindShift = 5;        // 0 single, 1 / 2 / 3: table of 4 / 8 / 16
+constexpr uint32_t kRingKindMask = 3u << kRingKindShift;
+constexpr uint32_t kRingLast = 1u << 7;       // last record of its run: apply
+constexpr uint32_t kRingNew = 1u << 8;        // first record of its coset: load
+constexpr uint32_t kRingFold = 1u << 9;       // complex64: fold the partial sums after this run
+constexpr uint32_t kRingFlipShift = 10;       // 4 bits: negate the loaded values of rows with this bit set
+constexpr uint32_t kRingFlipMask = 15u << kRingFlipShift;
+constexpr uint32_t kRingMaskShift = 14;       // 9 bits: m_lo
+
+constexpr uint32_t kRingFoldRuns = 16;        // complex64: runs per Kahan fold
+
+// Bytes of a record of each kind.
+constexpr uint32_t ring_record_bytes(uint32_t kind, uint32_t weight_bytes) {
+    return kind == 0 ? 16u : (kind == 1 ? 16u : 32u) + (weight_bytes << (kind + 1));
+}
+
 struct RingSchedule {
     uint32_t tile_bits = 0;
     uint32_t log_threads = 0;
     uint64_t cosets = 0;               // coset loads per output tile
+    uint64_t runs = 0;                 // runs per output tile
     uint32_t max_block_bytes = 0;      // largest step block
-    std::vector<uint32_t> step_info;   // d lo, d hi, block offset / 16, block bytes / 16
+    // 4 words per step: d, complex128 block offset / 16, complex64 block
+    // offset / 16, complex128 block bytes / 16 | complex64 block bytes / 16 << 16
+    std::vector<uint32_t> step_info;
     std::vector<uint8_t> blocks_c128;
     std::vector<uint8_t> blocks_c64;
 };
 
 constexpr uint32_t kRingBlockBytes = 8192;
+// A tile's row bits: thread bits [low, low + log_threads), register bits the
+// rest, bit 0 of the register index first (low = 1: row bit 0 is register bit 0).
+struct RingShapeBits {
+    uint32_t tile_bits, log_threads, low;
+};
+constexpr RingShapeBits kRingShapes[] = {{12, 9, 0}, {13, 9, 1}};
+constexpr int kRingShapeCount = 2;
+constexpr uint32_t kRingMaxZBits = 32;   // zs holds the z bits that are not register bits
 
-RingSchedule build_ring_schedule(const std::vector<MatrixTerm> &terms, uint32_t nqubits, uint32_t tile_bits,
-                                 uint32_t log_threads);
+// `c128`: with the complex128 blocks (the complex64 blocks are always built).
+RingSchedule build_ring_schedule(const std::vector<MatrixTerm> &terms, uint32_t nqubits, RingShapeBits shape,
+                                 bool c128 = true);
 
 constexpr uint32_t kBlockBytesMax = 16384;
 constexpr uint32_t kGroupRecBytes = 16;

@@ -227,71 +227,83 @@ __global__ void __launch_bounds__(kThreads, 1)
 
 // ------------------------------- ring kernel --------------------------------
 // k_ring: the tiled MVP with a ring of source tiles.
-//  * Sixteen warps own the output tile's 4096 rows (thread t: rows
-//    t + j * 512, j = 0..7) and keep their sums in registers.  Per step they
-//    wait for its stage ("full" mbarrier), walk its cosets -- one row-ordered
-//    load of 8 source values per coset -- and apply every group of the coset
-//    through a compile-time register permutation a (row j reads loaded value
-//    j ^ a).  Then each warp releases the stage with one arrive ("empty").
-//  * Thread 0 is also the producer: whenever a stage is released by every
-//    warp it has the TMA bulk-copy engine refill it with a later step's
-//    source tile (tile ^ d) and block.  It only tests the empty barriers
-//    (never waits on them), at each step and while its own warp waits for
-//    data, so no warp is set aside for issuing copies and no CTA-wide barrier
-//    runs after set-up: warps drift apart by up to the ring depth.
+//  * Sixteen warps own the output tile's rows and keep their sums in
+//    registers: 8 rows per thread (4096-row tiles) or, complex64 with enough
+//    tiles, 16 (8192-row tiles, kRingShapes).  Per step they wait for its stage
+//    ("full" mbarrier) and walk its records (ring_walk): one row-ordered load
+//    of the thread's source values per coset, one signed sum D and one
+//    multiply-add per row and run.  Then each warp releases the stage with one
+//    arrive ("empty").
+//  * What bounds it: neither HBM, shared memory nor the FMA pipes are full; a
+//    warp's chain of record load, sign, branch and multiply-adds is, with four
+//    warps per scheduler to hide it.  So the work per row counts: D is summed
+//    once per run and thread instead of multiplying every term into every row
+//    (2,000 random words on 28 qubits, complex128: 210 ms before, 190 now;
+//    Jordan-Wigner operator on 20 qubits: 30.7 before, 6.7 ms now), and 16 rows
+//    per thread halve the record walks per row (complex64, 26 qubits: 43.3 ms
+//    before, 38.4 with 8 rows, 26.3 with 16).  16 rows of complex64 with their
+//    Kahan sums would need 128 registers beside the 32 of the loaded values;
+//    the Kahan sums, touched every kRingFoldRuns runs only, live in tensor
+//    memory (64 columns per warp), which this kernel otherwise has no use for.
+//    256 threads of 16 rows in 4096-row tiles measured slower than 512 of 8
+//    (complex128 22.9 against 21.2 ms, complex64 19.7 against 18.1 ms, 25 qubits).
+//  * Refills: a producer warp (complex128) or the row warp that releases a
+//    stage last (complex64) has the TMA bulk-copy engine refill it with a later
+//    step's source tile (tile ^ d) and block; no CTA-wide barrier runs after
+//    set-up, so warps drift apart by up to the ring depth.
 //  * Every wait is bounded (2 s) and also ends when another thread raised the
-//    CTA's abort word; the kernel then records kErrTimeout, and thread 0
-//    waits (bounded) for the last fill of every stage before the block exits,
-//    so no copy is left writing into a finished block's memory.
+//    CTA's abort word; the kernel then records kErrTimeout, waits (bounded) for
+//    the last fill of every stage and frees its tensor memory before the block
+//    exits, so no copy is left writing into a finished block's memory.
 #ifdef TCP_DEBUG_BOUNDS
-// A block stays inside its `bytes`: header, coset records, group words and
-// the records they count; thread-bit masks below 512, permutations below 8.
-__device__ __forceinline__ bool ring_block_in_bounds(uint4 hdr, const uint4 *cos, const uint32_t *gw, uint32_t bytes) {
-    if (bytes > tcp::kRingBlockBytes || 16u + 16u * hdr.x + 4u * hdr.y > 16u * hdr.z || 16u * hdr.z > bytes) return false;
-    uint32_t groups = 0, records = 0;
-    for (uint32_t c = 0; c < hdr.x; ++c) {
-        if (cos[c].x >= 512u || cos[c].y != 0u) return false;
-        groups += cos[c].z;
+// The records of a block stay inside its `bytes`.
+template <typename R>
+__device__ __forceinline__ bool ring_block_in_bounds(const unsigned char *blk, uint32_t bytes) {
+    if (bytes < 16u || bytes + 16u > tcp::kRingBlockBytes) return false;
+    uint32_t at = 16u;
+    for (uint32_t n = *reinterpret_cast<const uint32_t *>(blk); n; --n) {
+        if (at + 16u > bytes) return false;
+        const uint32_t word = *reinterpret_cast<const uint32_t *>(blk + at + 4);
+        at += tcp::ring_record_bytes((word & tcp::kRingKindMask) >> tcp::kRingKindShift, sizeof(R));
     }
-    if (groups != hdr.y) return false;
-    for (uint32_t g = 0; g < groups; ++g) records += gw[g] >> 4;
-    return 16u * hdr.z + 16u * records <= bytes;
+    return at == bytes;
 }
 #endif
 
 // Issue the fill of ring step `i` (source tile and block) into its stage.
-template <typename R>
-__device__ __forceinline__ void ring_fill(const DevSchedule &s, const typename Cx<R>::T *__restrict__ x,
-                                          uint64_t tile, const uint4 *__restrict__ info, uint32_t i,
-                                          unsigned char *smem, uint64_t *full) {
-    constexpr uint32_t K = RingDepth<R>::K;
-    constexpr uint32_t TILE_BYTES = ring_tile_bytes<R>();
-    const uint32_t st = i % K;
-    const uint4 in = __ldg(&info[i]);
-    const uint64_t d = static_cast<uint64_t>(in.x) | (static_cast<uint64_t>(in.y) << 32);
-    const uint32_t blk_bytes = in.w * 16u;
-    unsigned char *dst = smem + st * ring_stage_bytes<R>();
+template <typename R, int SHAPE>
+__device__ __forceinline__ void ring_fill(const RingView &s, const typename Cx<R>::T *__restrict__ x, uint64_t tile,
+                                          const uint4 *__restrict__ info, uint32_t i, unsigned char *smem,
+                                          uint64_t *full) {
+    using G = RingGeo<R, SHAPE>;
+    const uint32_t st = i % G::kDepth;
+    const uint4 in = __ldg(&info[i]);  // see tcp::RingSchedule::step_info
+    const uint64_t d = in.x;
+    const uint32_t blk_off = sizeof(R) == 8 ? in.y : in.z;
+    const uint32_t blk_bytes = (sizeof(R) == 8 ? in.w & 0xffffu : in.w >> 16) * 16u;
+    unsigned char *dst = smem + st * G::kStageBytes;
     fence_proxy_async_smem();
-    mbar_arrive_expect_tx(&full[st], TILE_BYTES + blk_bytes);
-    bulk_copy_g2s(dst, x + ((tile ^ d) << kTileBitsC128), TILE_BYTES, &full[st]);
-    bulk_copy_g2s(dst + TILE_BYTES, ring_blocks<R>(s) + static_cast<size_t>(in.z) * 16u, blk_bytes, &full[st]);
+    mbar_arrive_expect_tx(&full[st], G::kTileBytes + blk_bytes);
+    bulk_copy_g2s(dst, x + ((tile ^ d) << G::kTileBits), G::kTileBytes, &full[st]);
+    bulk_copy_g2s(dst + G::kTileBytes, ring_blocks<R>(s) + static_cast<size_t>(blk_off) * 16u, blk_bytes, &full[st]);
 }
 
-template <typename R, bool PASSES, bool RHS_BLOCK = false>
-__global__ void __launch_bounds__(RingShape<R>::kThreadsPerCta, 1)
-    k_ring(DevSchedule s, const typename Cx<R>::T *__restrict__ x, typename Cx<R>::T *__restrict__ y,
+template <typename R, int SHAPE, bool PASSES, bool RHS_BLOCK = false>
+__global__ void __launch_bounds__(RingGeo<R, SHAPE>::kThreads, 1)
+    k_ring(RingView s, const typename Cx<R>::T *__restrict__ x, typename Cx<R>::T *__restrict__ y,
            int *__restrict__ err, uint64_t tile0, uint32_t pass, uint32_t accumulate, uint64_t rhs_stride) {
     using C = typename Cx<R>::T;
-    constexpr uint32_t K = RingDepth<R>::K;
-    constexpr uint32_t TILE_BYTES = ring_tile_bytes<R>();
-    constexpr uint32_t STAGE = ring_stage_bytes<R>();
-    constexpr bool kProducerWarp = RingShape<R>::kProducerWarp;
+    using G = RingGeo<R, SHAPE>;
+    constexpr uint32_t K = G::kDepth;
+    constexpr bool kProducerWarp = G::kProducerWarp;
+    constexpr int E = G::kRows;
     extern __shared__ __align__(128) unsigned char smem_raw[];
     __shared__ __align__(8) uint64_t full[K];
     __shared__ __align__(8) uint64_t empty[K];
     __shared__ uint32_t released[K];
     __shared__ uint32_t issued_end;
     __shared__ int abort_word;
+    __shared__ uint32_t tmem_base;
 
     const uint32_t tid = threadIdx.x;
     const uint32_t lane = tid & 31u;
@@ -303,36 +315,40 @@ __global__ void __launch_bounds__(RingShape<R>::kThreadsPerCta, 1)
         x += blockIdx.y * rhs_stride;
         y += blockIdx.y * rhs_stride;
     }
-    uint32_t step0 = 0, nsteps = s.ring_steps;
+    uint32_t step0 = 0, nsteps = s.steps;
     if constexpr (PASSES) {
         uint32_t b0, b1;
-        pass_range(s.ring_pass_begin, s.ring_pass_shift, tile, pass, b0, b1);
+        pass_range(s.pass_begin, s.pass_shift, tile, pass, b0, b1);
         step0 = b0;
         nsteps = b1 - b0;
     }
-    const uint4 *info = s.ring_info + step0;
+    const uint4 *info = s.info + step0;
     if (tid == 0) {
 #pragma unroll
         for (uint32_t k = 0; k < K; ++k) {
             mbar_init(&full[k], 1);
-            mbar_init(&empty[k], kRingWarps);
+            mbar_init(&empty[k], G::kWarps);
             released[k] = 0;
         }
         abort_word = 0;
         fence_mbar_init();
         if constexpr (!kProducerWarp) {
             const uint32_t first = nsteps < K ? nsteps : K;
-            for (uint32_t i = 0; i < first; ++i) ring_fill<R>(s, x, tile, info, i, smem_raw, full);
+            for (uint32_t i = 0; i < first; ++i) ring_fill<R, SHAPE>(s, x, tile, info, i, smem_raw, full);
             issued_end = first;
         }
+    }
+    if constexpr (G::kTmem) {
+        __syncwarp();
+        if (tid < 32u) tmem_alloc(&tmem_base, G::kTmemColumns);
     }
     __syncthreads();
     volatile int *abort_flag = &abort_word;
 
     if constexpr (kProducerWarp) {
-        if (tid >= kRingWarps * 32u) {
+        if (tid >= G::kWarps * 32u) {
             // ---------------- producer warp (lane 0 issues) ----------------
-            if (tid != kRingWarps * 32u) return;
+            if (tid != G::kWarps * 32u) return;
             uint32_t issued = 0;
             for (uint32_t st = 0; st < nsteps; ++st) {
                 if (st >= K && !mbar_wait_or_abort(&empty[st % K], ((st / K) - 1u) & 1u, abort_flag)) {
@@ -340,7 +356,7 @@ __global__ void __launch_bounds__(RingShape<R>::kThreadsPerCta, 1)
                     *abort_flag = 1;
                     break;
                 }
-                ring_fill<R>(s, x, tile, info, st, smem_raw, full);
+                ring_fill<R, SHAPE>(s, x, tile, info, st, smem_raw, full);
                 issued = st + 1;
             }
             // the last fill issued into each stage has landed before this returns
@@ -351,9 +367,11 @@ __global__ void __launch_bounds__(RingShape<R>::kThreadsPerCta, 1)
     }
 
     // ---------------- row warps ----------------
-    const uint32_t tile32 = static_cast<uint32_t>(tile);
-    RingAcc<R> acc[8];
-    uint32_t stage = 0, phase = 0, since = 0;
+    const uint32_t row_word = tid | (static_cast<uint32_t>(tile) << G::kLogT);
+    RingSums<R, SHAPE> sums;
+    if constexpr (G::kTmem) sums.init(tmem_base, tid >> 5);
+    uint32_t stage = 0, phase = 0;
+    bool failed = false;
     for (uint32_t st = 0; st < nsteps; ++st) {
         const bool landed = mbar_wait_or_abort(&full[stage], phase, abort_flag);
         if (__any_sync(0xffffffffu, !landed)) {
@@ -368,55 +386,20 @@ __global__ void __launch_bounds__(RingShape<R>::kThreadsPerCta, 1)
                         mbar_wait_bounded(&full[i % K], (i / K) & 1u);
                 }
             }
-            return;
+            failed = true;
+            break;
         }
-        const C *xs = reinterpret_cast<const C *>(smem_raw + stage * STAGE);
-        const unsigned char *blk = smem_raw + stage * STAGE + TILE_BYTES;
-        uint4 hdr = *reinterpret_cast<const uint4 *>(blk);
-        const uint4 *cos = reinterpret_cast<const uint4 *>(blk + 16);
-        const uint32_t *gw = reinterpret_cast<const uint32_t *>(blk + 16u + hdr.x * 16u);
-        const uint4 *trm = reinterpret_cast<const uint4 *>(blk + hdr.z * 16u);
+        const C *xs = reinterpret_cast<const C *>(smem_raw + stage * G::kStageBytes);
+        const unsigned char *blk = smem_raw + stage * G::kStageBytes + G::kTileBytes;
 #ifdef TCP_DEBUG_BOUNDS
         // debug builds check every block against its stage before walking it
         // and skip (recording kErrBounds) a block that would read outside it
-        if (!ring_block_in_bounds(hdr, cos, gw, __ldg(&info[st]).w * 16u)) {
+        const uint4 in = __ldg(&info[st]);
+        if (!ring_block_in_bounds<R>(blk, (sizeof(R) == 8 ? in.w & 0xffffu : in.w >> 16) * 16u)) {
             if (lane == 0u) atomicOr(err, kErrBounds);
-            hdr.x = 0u;
-        }
+        } else
 #endif
-        uint32_t g = 0;
-        for (uint32_t c = 0; c < hdr.x; ++c) {
-            const uint4 cr = cos[c];
-            C xv[8];
-            const C *src = xs + (tid ^ cr.x);
-#pragma unroll
-            for (int j = 0; j < 8; ++j) xv[j] = src[static_cast<uint32_t>(j) << kLogThreads];
-            for (uint32_t k = 0; k < cr.z; ++k, ++g) {
-                const uint32_t word = gw[g];
-                const uint32_t nt = word >> 4;
-                switch (word & 7u) {
-                case 0: ring_group<0, R>(trm, nt, tid, tile32, xv, acc); break;
-                case 1: ring_group<1, R>(trm, nt, tid, tile32, xv, acc); break;
-                case 2: ring_group<2, R>(trm, nt, tid, tile32, xv, acc); break;
-                case 3: ring_group<3, R>(trm, nt, tid, tile32, xv, acc); break;
-                case 4: ring_group<4, R>(trm, nt, tid, tile32, xv, acc); break;
-                case 5: ring_group<5, R>(trm, nt, tid, tile32, xv, acc); break;
-                case 6: ring_group<6, R>(trm, nt, tid, tile32, xv, acc); break;
-                default: ring_group<7, R>(trm, nt, tid, tile32, xv, acc); break;
-                }
-                trm += nt;
-                // FP32: fold the running partial sums into the compensated
-                // row sum every kRingCompensateGroups groups (counted across
-                // steps)
-                if constexpr (sizeof(R) == 4) {
-                    if (++since == kRingCompensateGroups) {
-                        since = 0;
-#pragma unroll
-                        for (int j = 0; j < 8; ++j) acc[j].compensate();
-                    }
-                }
-            }
-        }
+            ring_walk<R, SHAPE>(blk, xs, tid, row_word, sums);
         __syncwarp();
         if (lane == 0u) {
             if constexpr (kProducerWarp) {
@@ -426,11 +409,11 @@ __global__ void __launch_bounds__(RingShape<R>::kThreadsPerCta, 1)
                 // st + K: its reads, and every other warp's, are ordered
                 // before the counter update (fence), and the refill after it.
                 __threadfence_block();
-                if (atomicAdd(&released[stage], 1u) == kRingWarps - 1u) {
+                if (atomicAdd(&released[stage], 1u) == G::kWarps - 1u) {
                     released[stage] = 0u;
                     __threadfence_block();
                     if (st + K < nsteps) {
-                        ring_fill<R>(s, x, tile, info, st + K, smem_raw, full);
+                        ring_fill<R, SHAPE>(s, x, tile, info, st + K, smem_raw, full);
                         atomicMax(&issued_end, st + K + 1u);
                     }
                 }
@@ -441,20 +424,45 @@ __global__ void __launch_bounds__(RingShape<R>::kThreadsPerCta, 1)
             phase ^= 1u;
         }
     }
+    C *yt = y + (tile << G::kTileBits) + (tid << G::kLow);
+    if constexpr (G::kTmem) {
+        static_assert(G::kLow == 1, "rows 2 j and 2 j + 1 are adjacent");
+        __syncwarp();
+        if (!failed) {
+            sums.fold();
 #pragma unroll
-    for (int j = 0; j < 8; ++j) acc[j].compensate();
-    C *yt = y + (tile << kTileBitsC128);
-    if (accumulate) {
+            for (uint32_t k = 0; k < E / 4; ++k) {
+                float2 v[4];
+                sums.values(k, v);
 #pragma unroll
-        for (int j = 0; j < 8; ++j) {
-            C &out = yt[tid + (j << kLogThreads)];
-            const C v = acc[j].value();
-            out.x += v.x;
-            out.y += v.y;
+                for (uint32_t j = 0; j < 4; j += 2) {
+                    float4 *out = reinterpret_cast<float4 *>(yt + G::row(4 * k + j));
+                    float4 r = make_float4(v[j].x, v[j].y, v[j + 1].x, v[j + 1].y);
+                    if (accumulate) {
+                        const float4 o = *out;
+                        r = make_float4(o.x + r.x, o.y + r.y, o.z + r.z, o.w + r.w);
+                    }
+                    *out = r;
+                }
+            }
         }
+        __syncthreads();  // every warp is done with its tensor memory
+        if (tid < 32u) tmem_dealloc(tmem_base, G::kTmemColumns);
     } else {
+        if (failed) return;
+        sums.fold();
+        if (accumulate) {
 #pragma unroll
-        for (int j = 0; j < 8; ++j) yt[tid + (j << kLogThreads)] = acc[j].value();
+            for (int j = 0; j < E; ++j) {
+                C &out = yt[G::row(j)];
+                const C v = sums.value(j);
+                out.x += v.x;
+                out.y += v.y;
+            }
+        } else {
+#pragma unroll
+            for (int j = 0; j < E; ++j) yt[G::row(j)] = sums.value(j);
+        }
     }
 }
 
@@ -594,24 +602,23 @@ uint64_t chunk_start(uint64_t c, uint64_t tiles) {
     if (c + 1 == kHostChunks) return last + 3 * per / 4;
     return tiles;
 }
-constexpr uint64_t kHostChunkTiles = 8192;  // tiles from which the host apply is chunked
+constexpr uint64_t kHostChunkRows = uint64_t(1) << 25;  // rows from which the host apply is chunked
 
 size_t align_up(size_t v, size_t a) { return (v + a - 1) / a * a; }
 
 // Step ranges of the source-chunk passes (see DevSchedule::pass_begin): the
 // top kPassBits bits v of each step's outer pattern d, which is
 // non-decreasing in step order because steps are sorted by d.
-void set_passes(const std::vector<uint32_t> &step_info, uint32_t tile_bits, uint32_t nqubits, uint32_t *pass_begin,
+void set_passes(const std::vector<uint64_t> &pattern, uint32_t tile_bits, uint32_t nqubits, uint32_t *pass_begin,
                 uint32_t *pass_shift) {
-    const uint32_t nsteps = static_cast<uint32_t>(step_info.size() / 4);
+    const uint32_t nsteps = static_cast<uint32_t>(pattern.size());
     *pass_shift = kNoPasses;
     for (uint32_t v = 0; v <= kPassChunks; ++v) pass_begin[v] = v == 0 ? 0u : nsteps;
     if (tile_bits == 0 || nqubits < tile_bits + kPassBits) return;
     const uint32_t shift = nqubits - tile_bits - kPassBits;
     uint32_t prev = 0;
     for (uint32_t st = 0; st < nsteps; ++st) {
-        const uint64_t d = static_cast<uint64_t>(step_info[4 * st]) | (static_cast<uint64_t>(step_info[4 * st + 1]) << 32);
-        const uint32_t v = static_cast<uint32_t>(d >> shift);
+        const uint32_t v = static_cast<uint32_t>(pattern[st] >> shift);
         if (v >= kPassChunks || v < prev) return;  // not a sorted schedule: no passes
         for (uint32_t w = prev + 1; w <= v; ++w) pass_begin[w] = st;
         prev = v;
@@ -643,13 +650,21 @@ int upload(tcp_mvp_plan *p) {
         add(h.t_wf.data(), h.t_wf.size() * 4, reinterpret_cast<const void **>(&ds->dev.t_wf));
         ds->dev.nsteps = static_cast<uint32_t>(h.step_info.size() / 4);
         ds->dev.tile_bits = h.tile_bits;
-        set_passes(h.step_info, h.tile_bits, p->nqubits, ds->dev.pass_begin, &ds->dev.pass_shift);
-        tcp::RingSchedule &r = ds->ring;
-        add(r.step_info.data(), r.step_info.size() * 4, reinterpret_cast<const void **>(&ds->dev.ring_info));
-        add(r.blocks_c128.data(), r.blocks_c128.size(), reinterpret_cast<const void **>(&ds->dev.ring128));
-        add(r.blocks_c64.data(), r.blocks_c64.size(), reinterpret_cast<const void **>(&ds->dev.ring64));
-        ds->dev.ring_steps = static_cast<uint32_t>(r.step_info.size() / 4);
-        set_passes(r.step_info, r.tile_bits, p->nqubits, ds->dev.ring_pass_begin, &ds->dev.ring_pass_shift);
+        std::vector<uint64_t> pattern;  // outer pattern d of every step
+        for (size_t i = 0; i < h.step_info.size(); i += 4)
+            pattern.push_back(h.step_info[i] | static_cast<uint64_t>(h.step_info[i + 1]) << 32);
+        set_passes(pattern, h.tile_bits, p->nqubits, ds->dev.pass_begin, &ds->dev.pass_shift);
+        for (int shape = 0; shape < tcp::kRingShapeCount; ++shape) {
+            tcp::RingSchedule &r = ds->ring[shape];
+            RingView &v = ds->dev.ring[shape];
+            add(r.step_info.data(), r.step_info.size() * 4, reinterpret_cast<const void **>(&v.info));
+            add(r.blocks_c128.data(), r.blocks_c128.size(), reinterpret_cast<const void **>(&v.blocks128));
+            add(r.blocks_c64.data(), r.blocks_c64.size(), reinterpret_cast<const void **>(&v.blocks64));
+            v.steps = static_cast<uint32_t>(r.step_info.size() / 4);
+            pattern.clear();
+            for (size_t i = 0; i < r.step_info.size(); i += 4) pattern.push_back(r.step_info[i]);
+            set_passes(pattern, r.tile_bits, p->nqubits, v.pass_begin, &v.pass_shift);
+        }
         ds->dev.ngroups = static_cast<uint32_t>(h.g_mask.size());
     }
     size_t total = 256;  // error word first
@@ -696,40 +711,75 @@ template <int LOGE, typename R> int set_smem_attr() {
     return e == cudaSuccess ? TCP_OK : cuda_fail(e, "cudaFuncSetAttribute");
 }
 
-template <typename R> int set_ring_smem_attr() {
-    constexpr size_t bytes = ring_smem_bytes<R>();
-    cudaError_t e = cudaFuncSetAttribute(k_ring<R, false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                         static_cast<int>(bytes));
-    if (e == cudaSuccess)
-        e = cudaFuncSetAttribute(k_ring<R, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(bytes));
-    if (e == cudaSuccess)
-        e = cudaFuncSetAttribute(k_ring<R, false, true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                 static_cast<int>(bytes));
+template <typename K> int opt_in_smem(K *kernel, size_t bytes) {
+    cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(bytes));
     return e == cudaSuccess ? TCP_OK : cuda_fail(e, "cudaFuncSetAttribute");
 }
 
-// The ring kernel serves every plan with a ring schedule whose input the TMA
-// engine can address (16-byte aligned).
+template <typename R, int SHAPE> int set_ring_smem_attr() {
+    constexpr size_t bytes = RingGeo<R, SHAPE>::kSmemBytes;
+    int st = opt_in_smem(k_ring<R, SHAPE, false>, bytes);
+    if (st == TCP_OK) st = opt_in_smem(k_ring<R, SHAPE, true>, bytes);
+    if (st == TCP_OK) st = opt_in_smem(k_ring<R, SHAPE, false, true>, bytes);
+    return st;
+}
+
+// The ring kernel serves every plan with a ring schedule whose buffers the TMA
+// engine and 16-byte stores can address (16-byte aligned).
 bool ring_ok(const tcp_mvp_plan *p, const void *x) {
-    return p->sched.ring.tile_bits == kTileBitsC128 && p->nqubits >= kTileBitsC128 &&
+    return p->sched.ring[0].tile_bits == kTileBitsC128 && p->nqubits >= kTileBitsC128 &&
            (reinterpret_cast<uintptr_t>(x) % 16) == 0;
+}
+
+// Which shape serves `nrhs` vectors.  complex64 takes the 8192-row tiles (16
+// rows per thread: half the record walks per row) once they leave no SM idle
+// that 4096-row tiles would use: with 148 or fewer 4096-row tiles those run in
+// one wave, and twice the rows per block would take twice as long.
+template <typename R> int ring_shape(const tcp_mvp_plan *p, const void *y, uint32_t nrhs) {
+    if constexpr (sizeof(R) == 4) {
+        if (p->sched.ring[1].tile_bits && (p->dim >> kTileBitsC128) * nrhs > static_cast<uint64_t>(g_num_sms) &&
+            (reinterpret_cast<uintptr_t>(y) % 16) == 0)
+            return 1;
+    }
+    return 0;
+}
+
+// One ring launch of `tiles` output tiles from tile0 on, by `nrhs` vectors
+// (nrhs > 1: every tile, vectors `stride` apart).
+template <typename R, int SHAPE>
+void launch_ring(const tcp_mvp_plan *p, const void *x, void *y, int *err, cudaStream_t stream, uint64_t tile0,
+                 uint64_t tiles, int pass, bool accumulate, uint32_t nrhs) {
+    using C = typename Cx<R>::T;
+    using G = RingGeo<R, SHAPE>;
+    const RingView &v = p->sched.dev.ring[SHAPE];
+    const dim3 grid(static_cast<unsigned>(tiles), nrhs);
+    const auto *xc = static_cast<const C *>(x);
+    auto *yc = static_cast<C *>(y);
+    const uint32_t add = accumulate ? 1u : 0u;
+    if (pass >= 0)
+        k_ring<R, SHAPE, true><<<grid, G::kThreads, G::kSmemBytes, stream>>>(v, xc, yc, err, tile0,
+                                                                            static_cast<uint32_t>(pass), add, 0ull);
+    else if (nrhs > 1)
+        k_ring<R, SHAPE, false, true><<<grid, G::kThreads, G::kSmemBytes, stream>>>(v, xc, yc, err, tile0, 0u, add, p->dim);
+    else
+        k_ring<R, SHAPE, false><<<grid, G::kThreads, G::kSmemBytes, stream>>>(v, xc, yc, err, tile0, 0u, add, 0ull);
 }
 
 // Number of output tiles of the tiled kernels (0 when the plan uses the row
 // kernel for these buffers).
 template <typename R>
-uint64_t tiled_tiles(const tcp_mvp_plan *p, const void *x) {
+uint64_t tiled_tiles(const tcp_mvp_plan *p, const void *x, const void *y) {
     constexpr int LOGE = sizeof(R) == 8 ? kLogRowsC128 : kLogRowsC64;
     const uint32_t S = kLogThreads + LOGE;
     const bool aligned = (reinterpret_cast<uintptr_t>(x) % 16) == 0;
-    if (ring_ok(p, x)) return p->dim >> kTileBitsC128;
+    if (ring_ok(p, x)) return p->dim >> tcp::kRingShapes[ring_shape<R>(p, y, 1)].tile_bits;
     return (p->nqubits >= S && p->sched.host.tile_bits == S && aligned) ? (p->dim >> S) : 0;
 }
 
 // Whether the host path can split the state into kPassChunks parts for the
 // kernel that serves these buffers.
-bool has_passes(const tcp_mvp_plan *p, const void *x) {
-    return (ring_ok(p, x) ? p->sched.dev.ring_pass_shift : p->sched.dev.pass_shift) != kNoPasses;
+template <typename R> bool has_passes(const tcp_mvp_plan *p, const void *x, const void *y) {
+    return (ring_ok(p, x) ? p->sched.dev.ring[ring_shape<R>(p, y, 1)].pass_shift : p->sched.dev.pass_shift) != kNoPasses;
 }
 
 // Per-device, once: the shared-memory opt-in of the tiled kernels.
@@ -741,7 +791,10 @@ template <typename R> int ensure_smem_attrs(int device) {
     if (!attr_done[device]) {
         constexpr int LOGE = sizeof(R) == 8 ? kLogRowsC128 : kLogRowsC64;
         int st = set_smem_attr<LOGE, R>();
-        if (st == TCP_OK) st = set_ring_smem_attr<R>();
+        if (st == TCP_OK) st = set_ring_smem_attr<R, 0>();
+        if constexpr (sizeof(R) == 4) {
+            if (st == TCP_OK) st = set_ring_smem_attr<R, 1>();
+        }
         if (st != TCP_OK) return st;
         attr_done[device] = true;
     }
@@ -763,15 +816,12 @@ int launch_one(const tcp_mvp_plan *p, const void *x, void *y, cudaStream_t strea
     if (ring_ok(p, x)) {
         int st = ensure_smem_attrs<R>(p->device);
         if (st != TCP_OK) return st;
-        const uint64_t tiles = ntiles ? ntiles : (p->dim >> kTileBitsC128) - tile0;
-        const size_t smem = ring_smem_bytes<R>();
-        if (pass >= 0) {
-            k_ring<R, true><<<static_cast<unsigned>(tiles), RingShape<R>::kThreadsPerCta, smem, stream>>>(
-                ds.dev, static_cast<const C *>(x), static_cast<C *>(y), p->d_err, tile0, static_cast<uint32_t>(pass),
-                accumulate ? 1u : 0u, 0ull);
-        } else {
-            k_ring<R, false><<<static_cast<unsigned>(tiles), RingShape<R>::kThreadsPerCta, smem, stream>>>(
-                ds.dev, static_cast<const C *>(x), static_cast<C *>(y), p->d_err, tile0, 0u, accumulate ? 1u : 0u, 0ull);
+        const int shape = ring_shape<R>(p, y, 1);
+        const uint64_t tiles = ntiles ? ntiles : (p->dim >> tcp::kRingShapes[shape].tile_bits) - tile0;
+        if (shape == 0) {
+            launch_ring<R, 0>(p, x, y, p->d_err, stream, tile0, tiles, pass, accumulate, 1);
+        } else if constexpr (sizeof(R) == 4) {
+            launch_ring<R, 1>(p, x, y, p->d_err, stream, tile0, tiles, pass, accumulate, 1);
         }
     } else if (p->nqubits >= S && ds.host.tile_bits == S && aligned) {
         int st = ensure_smem_attrs<R>(p->device);
@@ -803,7 +853,7 @@ namespace tcp {
 // Whether `p` can run the ring kernel, with its shared-memory opt-in for the
 // dtype set up (outside any stream capture).
 int ring_prepare(const tcp_mvp_plan *p, bool c64) {
-    if (p->sched.ring.tile_bits != kTileBitsC128 || p->nqubits < kTileBitsC128)
+    if (p->sched.ring[0].tile_bits != kTileBitsC128 || p->nqubits < kTileBitsC128)
         return fail(TCP_ERR_INVALID_ARGUMENT, "the ring configuration needs a ring schedule (at least " +
                                                   std::to_string(kTileBitsC128) + " qubits) for every batch member");
     return c64 ? ensure_smem_attrs<float>(p->device) : ensure_smem_attrs<double>(p->device);
@@ -814,22 +864,20 @@ int ring_prepare(const tcp_mvp_plan *p, bool c64) {
 // wait is recorded in `err`.  Fails with TCP_ERR_INVALID_ARGUMENT when the
 // plan has no ring schedule or the buffers are not 16-byte aligned.
 int launch_ring_rhs(const tcp_mvp_plan *p, const void *x, void *y, uint32_t nrhs, bool c64, int *err,
-                    cudaStream_t stream) {
+                    cudaStream_t stream, bool accumulate) {
     if (!ring_ok(p, x) || (reinterpret_cast<uintptr_t>(y) % 16) != 0)
         return fail(TCP_ERR_INVALID_ARGUMENT, "the ring kernel needs a ring schedule and 16-byte aligned buffers");
     if (nrhs == 0 || nrhs > 65535u) return fail(TCP_ERR_INVALID_ARGUMENT, "RHS count out of range for one launch");
-    const dim3 grid(static_cast<unsigned>(p->dim >> kTileBitsC128), nrhs);
-    if (c64) {
-        int st = ensure_smem_attrs<float>(p->device);
-        if (st != TCP_OK) return st;
-        k_ring<float, false, true><<<grid, RingShape<float>::kThreadsPerCta, ring_smem_bytes<float>(), stream>>>(
-            p->sched.dev, static_cast<const float2 *>(x), static_cast<float2 *>(y), err, 0ull, 0u, 0u, p->dim);
-    } else {
-        int st = ensure_smem_attrs<double>(p->device);
-        if (st != TCP_OK) return st;
-        k_ring<double, false, true><<<grid, RingShape<double>::kThreadsPerCta, ring_smem_bytes<double>(), stream>>>(
-            p->sched.dev, static_cast<const double2 *>(x), static_cast<double2 *>(y), err, 0ull, 0u, 0u, p->dim);
-    }
+    int st = c64 ? ensure_smem_attrs<float>(p->device) : ensure_smem_attrs<double>(p->device);
+    if (st != TCP_OK) return st;
+    const int shape = c64 ? ring_shape<float>(p, y, nrhs) : 0;
+    const uint64_t tiles = p->dim >> tcp::kRingShapes[shape].tile_bits;
+    if (!c64)
+        launch_ring<double, 0>(p, x, y, err, stream, 0, tiles, -1, accumulate, nrhs);
+    else if (shape == 0)
+        launch_ring<float, 0>(p, x, y, err, stream, 0, tiles, -1, accumulate, nrhs);
+    else
+        launch_ring<float, 1>(p, x, y, err, stream, 0, tiles, -1, accumulate, nrhs);
     cudaError_t e = cudaGetLastError();
     return e == cudaSuccess ? TCP_OK : cuda_fail(e, "ring kernel launch");
 }
@@ -1099,9 +1147,9 @@ int apply_host(const tcp_mvp_plan *plan, const R *state, uint64_t state_len, R *
     // Every launch is queued right after the copy it waits for; ordinary
     // (pageable) buffers move through the staging ring (HostCopies).  Smaller
     // applies copy, launch once and copy back on one stream.
-    const uint64_t tiles = tiled_tiles<R>(plan, ws.x);
-    const uint64_t chunks = tiles >= kHostChunkTiles ? kHostChunks : 1;
-    const bool passes = chunks > 1 && has_passes(plan, ws.x);
+    const uint64_t tiles = tiled_tiles<R>(plan, ws.x, ws.y);
+    const uint64_t chunks = tiles > 0 && plan->dim >= kHostChunkRows ? kHostChunks : 1;
+    const bool passes = chunks > 1 && has_passes<R>(plan, ws.x, ws.y);
     // Source parts in eighths of the state's tiles: the input goes in as
     // eighth 0, eighth 1, the second quarter and the second half; pass k
     // reads exactly part k (kHostPass: base part | log2(parts) << 4), so the
@@ -1253,7 +1301,8 @@ extern "C" int tcp_mvp_plan_create(uint32_t nqubits, uint64_t term_count, uint32
     {
         tcp::Range range("tile schedules");
         p->sched.host = tcp::build_schedule(p->terms, nqubits, kTileBitsC128, kLogThreads);
-        p->sched.ring = tcp::build_ring_schedule(p->terms, nqubits, kTileBitsC128, kLogThreads);
+        p->sched.ring[0] = tcp::build_ring_schedule(p->terms, nqubits, tcp::kRingShapes[0]);
+        p->sched.ring[1] = tcp::build_ring_schedule(p->terms, nqubits, tcp::kRingShapes[1], false);
     }
     st = upload(p.get());
     if (st) return st;
@@ -1301,8 +1350,8 @@ extern "C" int tcp_mvp_plan_info(const tcp_mvp_plan *plan, tcp_mvp_plan_info_t *
     info->log_threads = plan->sched.host.log_threads;
     info->steps = plan->sched.host.step_info.size() / 4;
     info->outer_patterns = plan->sched.host.distinct_outer;
-    info->ring_steps = plan->sched.ring.step_info.size() / 4;
-    info->cosets = plan->sched.ring.cosets;
+    info->ring_steps = plan->sched.ring[0].step_info.size() / 4;
+    info->cosets = plan->sched.ring[0].cosets;
     return TCP_OK;
 }
 
@@ -1331,6 +1380,9 @@ int apply_device(const tcp_mvp_plan *plan, const void *d_state, void *d_result, 
     const size_t bytes = static_cast<size_t>(len) * elem * nrhs;
     if (overlaps(d_state, d_result, bytes)) return fail(TCP_ERR_INVALID_ARGUMENT, "input and output must not overlap");
     cudaStream_t s = static_cast<cudaStream_t>(stream);
+    // a block of vectors: one ring launch over tiles x vectors
+    if (nrhs > 1 && nrhs <= 65535u && ring_ok(plan, d_state) && (reinterpret_cast<uintptr_t>(d_result) % 16) == 0)
+        return tcp::launch_ring_rhs(plan, d_state, d_result, nrhs, dtype == TCP_DTYPE_C64, plan->d_err, s, accumulate);
     for (uint32_t v = 0; v < nrhs; ++v) {
         const void *x = static_cast<const unsigned char *>(d_state) + static_cast<size_t>(v) * len * elem;
         void *y = static_cast<unsigned char *>(d_result) + static_cast<size_t>(v) * len * elem;
@@ -1515,8 +1567,7 @@ extern "C" int tcp_mvp_apply_into_host_noalloc(const tcp_mvp_plan *plan, const d
     const tcp::DeviceSchedule &ds = plan->sched;
     const uint32_t S = kTileBitsC128;
     if (ring_ok(plan, dx)) {
-        k_ring<double, false><<<static_cast<unsigned>(plan->dim >> S), RingShape<double>::kThreadsPerCta, ring_smem_bytes<double>(), s>>>(
-            ds.dev, dx, dy, d_status, 0, 0u, 0u, 0ull);
+        launch_ring<double, 0>(plan, dx, dy, d_status, s, 0, plan->dim >> S, -1, false, 1);
     } else if (plan->nqubits >= S && ds.host.tile_bits == S) {
         const size_t smem = tiled_smem_bytes<kLogRowsC128, double>();
         k_tiled<kLogRowsC128, double, false><<<static_cast<unsigned>(plan->dim >> S), kThreads, smem, s>>>(

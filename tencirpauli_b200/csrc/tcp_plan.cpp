@@ -8,6 +8,8 @@
 #include <cstring>
 #include <map>
 #include <numeric>
+#include <tuple>
+#include <unordered_map>
 
 #include "tcp_internal.h"
 
@@ -249,158 +251,326 @@ Schedule build_schedule(const std::vector<MatrixTerm> &terms, uint32_t nqubits, 
     return s;
 }
 
-RingSchedule build_ring_schedule(const std::vector<MatrixTerm> &terms, uint32_t nqubits, uint32_t tile_bits,
-                                 uint32_t log_threads) {
+namespace {
+
+struct SignedWeight {
+    uint32_t zs;
+    double w;
+};
+
+// Terms in one affine space z0 ^ span(v[0 .. rank)): the table of their signed
+// sums over the rank index bits.
+struct SignTable {
+    uint32_t z0 = 0;
+    uint32_t v[4] = {0, 0, 0, 0};
+    uint32_t rank = 0;
+    double t[16] = {};
+};
+
+// Coordinates of zs ^ z0 in a growing basis of at most 4 vectors; returns
+// false when it lies outside and the basis is full.
+struct AffineSpan {
+    uint32_t z0 = 0;
+    uint32_t v[4] = {0, 0, 0, 0};       // the basis as given
+    uint32_t red[4] = {0, 0, 0, 0};     // reduced vectors
+    uint32_t combo[4] = {0, 0, 0, 0};   // each as a combination of v
+    uint32_t rank = 0;
+    bool coordinates(uint32_t zs, uint32_t max_rank, uint32_t &coord) {
+        uint32_t x = zs ^ z0, c = 0;
+        for (uint32_t k = 0; k < rank; ++k) {
+            if ((x ^ red[k]) < x) {  // red[k]'s top bit is set in x
+                x ^= red[k];
+                c ^= combo[k];
+            }
+        }
+        if (x != 0) {
+            if (rank == max_rank) return false;
+            v[rank] = zs ^ z0;
+            // keep the reduced vectors in descending order of their top bit
+            uint32_t r = x, rc = c ^ (1u << rank);
+            uint32_t at = rank;
+            while (at > 0 && red[at - 1] < r) {
+                red[at] = red[at - 1];
+                combo[at] = combo[at - 1];
+                --at;
+            }
+            red[at] = r;
+            combo[at] = rc;
+            c = 1u << rank;
+            ++rank;
+        }
+        coord = c;
+        return true;
+    }
+};
+
+// Fewest terms for which a table of rank r is taken instead of singles: per
+// thread a single takes about 8 instructions, a table of rank 2, 3, 4 about
+// 18, 24 and 28.
+constexpr size_t kTableMinTerms[5] = {3, 3, 3, 4, 5};
+
+void fill_table(const AffineSpan &span, const std::vector<SignedWeight> &terms, const std::vector<uint32_t> &coords,
+                SignTable &out) {
+    out.z0 = span.z0;
+    out.rank = span.rank;
+    for (uint32_t k = 0; k < 4; ++k) out.v[k] = k < span.rank ? span.v[k] : 0u;
+    for (uint32_t i = 0; i < 16u; ++i) {
+        double sum = 0.0;
+        for (size_t k = 0; k < terms.size(); ++k)
+            sum += (__builtin_popcount(coords[k] & i) & 1) ? -terms[k].w : terms[k].w;
+        out.t[i] = sum;
+    }
+}
+
+// Cut the terms of one run into singles and tables.  Whole runs of affine
+// rank <= 4 become one table; larger ones are covered greedily by tables of
+// rank 4, each grown direction by direction to cover the most remaining terms.
+void tabulate(std::vector<SignedWeight> rest, std::vector<SignedWeight> &singles, std::vector<SignTable> &tables) {
+    while (rest.size() >= kTableMinTerms[2]) {
+        AffineSpan span;
+        std::vector<uint32_t> coords;
+        std::vector<SignedWeight> in, out;
+        span.z0 = rest[0].zs;
+        bool whole = true;
+        for (const SignedWeight &s : rest) {
+            uint32_t c;
+            if (!span.coordinates(s.zs, 4, c)) {
+                whole = false;
+                break;
+            }
+            coords.push_back(c);
+        }
+        if (whole) {
+            in.swap(rest);
+        } else {
+            std::unordered_map<uint32_t, uint32_t> left;  // zs -> position
+            left.reserve(rest.size() * 2);
+            for (size_t i = 0; i < rest.size(); ++i) left.emplace(rest[i].zs, static_cast<uint32_t>(i));
+            AffineSpan best;
+            size_t best_count = 0;
+            for (const uint32_t z0 : {rest[0].zs, 0u}) {
+                AffineSpan cur;
+                cur.z0 = z0;
+                std::vector<uint32_t> points{z0};
+                size_t covered = left.count(z0);
+                for (uint32_t dim = 0; dim < 4; ++dim) {
+                    uint32_t best_v = 0;
+                    size_t best_new = 0;
+                    const size_t stride = std::max<size_t>(1, rest.size() / 32);
+                    for (size_t i = 0; i < rest.size(); i += stride) {
+                        const uint32_t v = rest[i].zs ^ z0;
+                        AffineSpan probe = cur;
+                        uint32_t c;
+                        probe.coordinates(rest[i].zs, 4, c);
+                        if (probe.rank == cur.rank) continue;  // already covered
+                        size_t fresh = 0;
+                        for (uint32_t p : points) fresh += left.count(p ^ v);
+                        if (fresh > best_new) {
+                            best_new = fresh;
+                            best_v = v;
+                        }
+                    }
+                    if (best_new == 0) break;
+                    uint32_t c;
+                    cur.coordinates(z0 ^ best_v, 4, c);
+                    const size_t n = points.size();
+                    for (size_t i = 0; i < n; ++i) points.push_back(points[i] ^ best_v);
+                    covered += best_new;
+                }
+                if (covered > best_count) {
+                    best_count = covered;
+                    best = cur;
+                }
+            }
+            if (best_count < kTableMinTerms[best.rank]) break;
+            span = best;
+            coords.clear();
+            for (const SignedWeight &s : rest) {
+                uint32_t c;
+                if (span.rank > 0 && span.coordinates(s.zs, span.rank, c)) {
+                    in.push_back(s);
+                    coords.push_back(c);
+                } else {
+                    out.push_back(s);
+                }
+            }
+            rest.swap(out);
+        }
+        if (in.size() < kTableMinTerms[span.rank]) {
+            singles.insert(singles.end(), in.begin(), in.end());
+            continue;
+        }
+        SignTable t;
+        fill_table(span, in, coords, t);
+        tables.push_back(t);
+    }
+    singles.insert(singles.end(), rest.begin(), rest.end());
+}
+
+}  // namespace
+
+RingSchedule build_ring_schedule(const std::vector<MatrixTerm> &terms, uint32_t nqubits, RingShapeBits shape, bool c128) {
     RingSchedule r;
-    // The ring kernel covers 512 threads x 8 rows per tile, and outer z bits
-    // that fit 32 bits.
-    if (log_threads != 9 || tile_bits != 12 || nqubits < tile_bits || nqubits - tile_bits > 32) return r;
-    const uint32_t S = tile_bits, L = log_threads;
-    const uint64_t inner = (1ull << S) - 1, tmask = (1ull << L) - 1;
+    const uint32_t S = shape.tile_bits, L = shape.log_threads;
+    if (nqubits < S || nqubits - (S - L) > kRingMaxZBits) return r;
+    const uint64_t inner = (1ull << S) - 1;
+    const uint32_t tmask = (1u << L) - 1u, lowmask = (1u << shape.low) - 1u;
+    auto thread_part = [&](uint64_t m) { return static_cast<uint32_t>(m >> shape.low) & tmask; };
+    auto row_part = [&](uint64_t m) {
+        const uint32_t high = static_cast<uint32_t>((m & inner) >> (shape.low + L));
+        return (static_cast<uint32_t>(m) & lowmask) | (high << shape.low);
+    };
     r.tile_bits = S;
     r.log_threads = L;
 
-    // One record per real or imaginary weight part; canonical order inside a
-    // group, real part before imaginary part.
+    // One item per real or imaginary weight part; canonical order inside a run.
     struct Item {
-        uint64_t d;
-        uint32_t m_lo, jh;
-        uint64_t mask;
-        uint64_t z;
+        uint32_t d, m_lo, jh, imag, zj, zs;
         uint64_t canon;
-        uint32_t imag;
-        double w;
+        double w;  // folded
     };
     std::vector<Item> items;
     items.reserve(terms.size() + 8);
     for (uint64_t i = 0; i < terms.size(); ++i) {
         const MatrixTerm &t = terms[i];
-        const uint64_t d = t.x_mask >> S;
-        const uint32_t m_lo = static_cast<uint32_t>(t.x_mask & tmask);
-        const uint32_t jh = static_cast<uint32_t>((t.x_mask & inner) >> L);
-        if (t.w_re != 0.0 || t.w_im == 0.0) items.push_back({d, m_lo, jh, t.x_mask, t.z_mask, i, 0u, t.w_re});
-        if (t.w_im != 0.0) items.push_back({d, m_lo, jh, t.x_mask, t.z_mask, i, 1u, t.w_im});
-    }
-    std::stable_sort(items.begin(), items.end(), [](const Item &a, const Item &b) {
-        if (a.d != b.d) return a.d < b.d;
-        if (a.m_lo != b.m_lo) return a.m_lo < b.m_lo;
-        if (a.jh != b.jh) return a.jh < b.jh;
-        return a.canon < b.canon;
-    });
-
-    struct PGroup {
-        uint32_t a = 0;
-        std::vector<size_t> items;
-    };
-    struct PCoset {
-        uint32_t m_lo = 0, jh = 0;
-        std::vector<PGroup> groups;
-    };
-    auto pattern_of = [&](const Item &it) {
-        const uint32_t zj = static_cast<uint32_t>((it.z & inner) >> L);
-        uint32_t pattern = 0;
-        for (uint32_t j = 0; j < 8; ++j) pattern |= (static_cast<uint32_t>(__builtin_popcount(zj & j)) & 1u) << j;
-        return pattern;
-    };
-    // run of a record: real / imaginary weight x uniform / patterned sign
-    auto run_of = [&](const Item &it) { return (it.imag << 1) | (pattern_of(it) != 0u ? 1u : 0u); };
-    std::vector<PCoset> pend;
-    size_t pend_groups = 0, pend_terms = 0;
-    uint64_t cur_d = 0;
-    auto block_bytes = [](size_t c, size_t g, size_t t) { return 16 + 16 * c + (4 * g + 15) / 16 * 16 + 16 * t; };
-    auto flush = [&]() {
-        if (pend.empty()) return;
-        const size_t off = r.blocks_c128.size();
-        const size_t terms_off = 16 + 16 * pend.size() + (4 * pend_groups + 15) / 16 * 16;
-        put(r.blocks_c128, static_cast<uint32_t>(pend.size()));
-        put(r.blocks_c128, static_cast<uint32_t>(pend_groups));
-        put(r.blocks_c128, static_cast<uint32_t>(terms_off / 16));
-        put(r.blocks_c128, uint32_t(0));
-        for (auto &c : pend) {
-            put(r.blocks_c128, c.m_lo);
-            put(r.blocks_c128, c.jh);
-            put(r.blocks_c128, static_cast<uint32_t>(c.groups.size()));
-            put(r.blocks_c128, uint32_t(0));
+        Item it;
+        it.d = static_cast<uint32_t>(t.x_mask >> S);
+        it.m_lo = thread_part(t.x_mask);
+        it.jh = row_part(t.x_mask);
+        const uint32_t zlo = thread_part(t.z_mask), zt = static_cast<uint32_t>(t.z_mask >> S);
+        it.zj = row_part(t.z_mask);
+        it.zs = zlo | (zt << L);
+        it.canon = i;
+        const bool flip = ((__builtin_popcount(zt & it.d) + __builtin_popcount(zlo & it.m_lo)) & 1) != 0;
+        for (uint32_t imag = 0; imag < 2; ++imag) {
+            const double w = imag ? t.w_im : t.w_re;
+            if (imag ? w == 0.0 : (w == 0.0 && t.w_im != 0.0)) continue;
+            it.imag = imag;
+            it.w = flip ? -w : w;
+            items.push_back(it);
         }
-        for (auto &c : pend)
-            for (auto &g : c.groups) put(r.blocks_c128, g.a | static_cast<uint32_t>(g.items.size() << 4));
-        while ((r.blocks_c128.size() - off) % 16) r.blocks_c128.push_back(0);
-        for (auto &c : pend) {
-            for (auto &g : c.groups) {
-                // records of a group in four runs: real uniform-sign, real
-                // patterned, imaginary uniform-sign, imaginary patterned
-                std::stable_sort(g.items.begin(), g.items.end(),
-                                 [&](size_t u, size_t v) { return run_of(items[u]) < run_of(items[v]); });
-                for (size_t k : g.items) {
-                    const Item &it = items[k];
-                    const uint64_t zt = it.z >> S;
-                    const uint32_t zlo = static_cast<uint32_t>(it.z & tmask);
-                    const uint32_t zj = static_cast<uint32_t>((it.z & inner) >> L);
-                    const uint32_t pattern = pattern_of(it);
-                    const bool flip = ((__builtin_popcountll(zt & cur_d) + __builtin_popcount(zlo & it.m_lo) +
-                                        __builtin_popcount(zj & it.jh)) & 1) != 0;
-                    const double w = flip ? -it.w : it.w;
-                    put(r.blocks_c128, zlo | (pattern << 9) | (it.imag << 17));
-                    put(r.blocks_c128, static_cast<uint32_t>(zt));
-                    put(r.blocks_c128, w);
+    }
+    // Inside a coset the row parts zj come in Gray-code order, so that most
+    // changes flip the rows of one bit.
+    auto gray_rank = [](uint32_t zj) { return zj ^ (zj >> 1) ^ (zj >> 2) ^ (zj >> 3); };
+    auto key = [&](const Item &a) {
+        return std::make_tuple(a.d, a.m_lo, gray_rank(a.zj), a.jh, a.imag, a.canon);
+    };
+    std::sort(items.begin(), items.end(), [&](const Item &a, const Item &b) { return key(a) < key(b); });
+
+    std::vector<uint8_t> out128, out64;  // records of the open step
+    const uint32_t wb = c128 ? 8u : 4u;  // weight bytes of the larger blocks
+    uint32_t count = 0, cur_d = 0, cur_zj = 0, run_index = 0;
+    int64_t cur_coset = -1;              // m_lo of the open coset (-1: none)
+    auto flush = [&]() {
+        if (count == 0) return;
+        const size_t off[2] = {r.blocks_c128.size(), r.blocks_c64.size()};
+        size_t bytes[2] = {0, 0};
+        for (int f = c128 ? 0 : 1; f < 2; ++f) {
+            std::vector<uint8_t> &dst = f ? r.blocks_c64 : r.blocks_c128;
+            put(dst, count);
+            for (int k = 0; k < 3; ++k) put(dst, uint32_t(0));
+            const std::vector<uint8_t> &src = f ? out64 : out128;
+            dst.insert(dst.end(), src.begin(), src.end());
+            bytes[f] = dst.size() - off[f];
+        }
+        r.max_block_bytes = std::max<uint32_t>(r.max_block_bytes, static_cast<uint32_t>(bytes[c128 ? 0 : 1]));
+        r.step_info.push_back(cur_d);
+        r.step_info.push_back(static_cast<uint32_t>(off[0] / 16));
+        r.step_info.push_back(static_cast<uint32_t>(off[1] / 16));
+        r.step_info.push_back(static_cast<uint32_t>(bytes[0] / 16) | static_cast<uint32_t>(bytes[1] / 16) << 16);
+        out128.clear();
+        out64.clear();
+        count = 0;
+        cur_coset = -1;
+    };
+    // `record` in both precisions; zs or z0, word, then the kind's content.
+    auto put_record = [&](uint32_t kind, uint32_t zs, uint32_t word, const SignTable *t, double w) {
+        for (int f = c128 ? 0 : 1; f < 2; ++f) {
+            std::vector<uint8_t> &dst = f ? out64 : out128;
+            auto weight = [&](double v) {
+                if (f)
+                    put(dst, static_cast<float>(v));
+                else
+                    put(dst, v);
+            };
+            put(dst, zs);
+            put(dst, word | (kind << kRingKindShift));
+            if (kind == 0) {
+                weight(w);
+                if (f) put(dst, uint32_t(0));
+                continue;
+            }
+            put(dst, t->v[0]);
+            put(dst, t->v[1]);
+            if (kind > 1) {
+                put(dst, t->v[2]);
+                put(dst, kind > 2 ? t->v[3] : 0u);
+                put(dst, uint64_t(0));
+            }
+            for (uint32_t k = 0; k < (2u << kind); ++k) weight(t->t[k]);
+        }
+        ++count;
+    };
+    for (size_t k = 0; k < items.size();) {
+        const Item &first = items[k];
+        if (k == 0 || first.d != cur_d) {
+            flush();
+            cur_d = first.d;
+        }
+        std::vector<SignedWeight> list;
+        size_t e = k;
+        for (; e < items.size(); ++e) {
+            const Item &it = items[e];
+            if (it.d != first.d || it.m_lo != first.m_lo || it.jh != first.jh || it.imag != first.imag ||
+                it.zj != first.zj)
+                break;
+            list.push_back({it.zs, it.w});
+        }
+        std::vector<SignedWeight> singles;
+        std::vector<SignTable> tables;
+        tabulate(std::move(list), singles, tables);
+        // The run's records in order, a run per stretch that fits the block.
+        const uint32_t run_word = first.jh | (first.imag ? kRingImag : 0u) | (first.m_lo << kRingMaskShift);
+        const size_t total = singles.size() + tables.size();
+        auto kind_of = [&](size_t i) {
+            return i < singles.size() ? 0u : std::max<uint32_t>(2u, tables[i - singles.size()].rank) - 1u;
+        };
+        // header, the records so far, `bytes` more and the 16 unused bytes
+        auto room = [&](uint32_t bytes) {
+            return 16 + (c128 ? out128 : out64).size() + bytes + 16 <= kRingBlockBytes;
+        };
+        for (size_t i = 0; i < total; ++i) {
+            const uint32_t kind = kind_of(i);
+            if (!room(ring_record_bytes(kind, wb))) flush();
+            uint32_t word = run_word;
+            if (cur_coset != static_cast<int64_t>(first.m_lo)) {
+                word |= kRingNew;
+                cur_coset = first.m_lo;
+                cur_zj = 0;
+                ++r.cosets;
+            }
+            word |= (first.zj ^ cur_zj) << kRingFlipShift;
+            cur_zj = first.zj;
+            const bool ends = i + 1 == total;
+            // the run also ends where the next record would open another step
+            const bool cut = !ends && !room(ring_record_bytes(kind, wb) + ring_record_bytes(kind_of(i + 1), wb));
+            if (ends || cut) {
+                word |= kRingLast;
+                ++r.runs;
+                if (++run_index % kRingFoldRuns == 0) {
+                    word |= kRingFold;
+                    cur_coset = -1;
                 }
             }
+            if (i < singles.size())
+                put_record(kind, singles[i].zs, word, nullptr, singles[i].w);
+            else
+                put_record(kind, tables[i - singles.size()].z0, word, &tables[i - singles.size()], 0.0);
         }
-        const size_t bytes = r.blocks_c128.size() - off;
-        r.max_block_bytes = std::max<uint32_t>(r.max_block_bytes, static_cast<uint32_t>(bytes));
-        r.step_info.push_back(static_cast<uint32_t>(cur_d));
-        r.step_info.push_back(static_cast<uint32_t>(cur_d >> 32));
-        r.step_info.push_back(static_cast<uint32_t>(off / 16));
-        r.step_info.push_back(static_cast<uint32_t>(bytes / 16));
-        r.cosets += pend.size();
-        pend.clear();
-        pend_groups = pend_terms = 0;
-    };
-    bool have = false;
-    for (size_t k = 0; k < items.size(); ++k) {
-        const Item &it = items[k];
-        if (!have || it.d != cur_d) {
-            flush();
-            cur_d = it.d;
-            have = true;
-        }
-        bool new_coset = pend.empty() || pend.back().m_lo != it.m_lo;
-        bool new_group = new_coset || items[pend.back().groups.back().items.back()].mask != it.mask;
-        if (block_bytes(pend.size() + new_coset, pend_groups + new_group, pend_terms + 1) > kRingBlockBytes) {
-            flush();
-            new_coset = new_group = true;
-        }
-        if (new_coset) {
-            PCoset c;
-            c.m_lo = it.m_lo;
-            c.jh = 0;  // row-order loads: the permutation lives in each group's a
-            pend.push_back(c);
-        }
-        if (new_group) {
-            PGroup g;
-            g.a = it.jh;
-            pend.back().groups.push_back(g);
-            ++pend_groups;
-        }
-        pend.back().groups.back().items.push_back(k);
-        ++pend_terms;
+        k = e;
     }
     flush();
-    // complex64 blocks: the same layout with the weight rounded to FP32
-    r.blocks_c64 = r.blocks_c128;
-    for (size_t i = 0; i + 4 <= r.step_info.size(); i += 4) {
-        const size_t off = static_cast<size_t>(r.step_info[i + 2]) * 16;
-        const size_t bytes = static_cast<size_t>(r.step_info[i + 3]) * 16;
-        uint32_t terms_off;
-        std::memcpy(&terms_off, &r.blocks_c128[off + 8], 4);
-        for (size_t p = off + static_cast<size_t>(terms_off) * 16; p < off + bytes; p += 16) {
-            double w;
-            std::memcpy(&w, &r.blocks_c128[p + 8], 8);
-            const float f = static_cast<float>(w);
-            std::memcpy(&r.blocks_c64[p + 8], &f, 4);
-            std::memset(&r.blocks_c64[p + 12], 0, 4);
-        }
-    }
     return r;
 }
 

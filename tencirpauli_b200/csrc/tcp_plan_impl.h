@@ -13,7 +13,7 @@ namespace tcp {
 
 struct DeviceSchedule {
     Schedule host;
-    RingSchedule ring;  // k_ring's schedule (tile_bits = 0: the plan does not use it)
+    RingSchedule ring[kRingShapeCount];  // k_ring's schedules (tile_bits = 0: the plan has none of this shape)
     tcpdev::DevSchedule dev{};
 };
 
@@ -65,5 +65,5 @@ int length_error(uint64_t expected, uint64_t actual);
 bool overlaps(const void *a, const void *b, size_t bytes);
 int ring_prepare(const tcp_mvp_plan *p, bool c64);
 int launch_ring_rhs(const tcp_mvp_plan *p, const void *x, void *y, uint32_t nrhs, bool c64, int *err,
-                    cudaStream_t stream);
+                    cudaStream_t stream, bool accumulate = false);
 }  // namespace tcp
