@@ -36,6 +36,7 @@
 #include <memory>
 #include <mutex>
 #include <string>
+#include <type_traits>
 #include <unordered_map>
 #include <vector>
 
@@ -307,6 +308,11 @@ struct U1Apply {
     const float2 *awf;     // [ta]
     const double2 *diag;   // [dim] or null when there is no x == 0 group
     uint32_t na, nb, nc, ta;
+    // Pair view (k_u1_pairs): records {x, z_out, C} (f64, or f32 and 0) in six
+    // classes, class q in [pair_seg[q], pair_seg[q + 1]); null when the plan
+    // has other groups.
+    const uint4 *pairs, *pairsf;
+    uint32_t pair_seg[7];
 };
 
 template <typename R> struct Cplx;
@@ -543,6 +549,106 @@ __global__ void __launch_bounds__(kU1Threads) k_u1_apply(U1Dev p, U1Apply a, siz
             for (int u = 0; u < U; ++u)
                 if (live[u]) cmac<R, C>(ar, ai, cr, ci, vr[u], vi[u], xv[u]);
         }
+        C out;
+        out.x = ar;
+        out.y = ai;
+        y[i] = out;
+    }
+}
+
+// y = H_sector x when every group is a real constant on one pair of qubits
+// (exchange, hopping): the usual lattice and one-body operators.  A pair is
+// live where its two bits differ, and a live group is one multiply-add by
+// +-C.  Against the general kernel this drops, per row and group, the popcount
+// of the live test, the complex product of a real constant and the branch
+// around a dead group (whose value is not loaded, and added as 0 C); and with
+// two-level ranks a pair inside the low (high) half of the state changes one
+// table lookup only, so the groups are sorted into classes: low, high, both,
+// each without and with a sign mask z_out.  What remains is issue and the
+// gathers from L2 (4 x 6 J1-J2 half filling, complex128: 376 us before, 268
+// now; 4 groups in flight 273, 8 at 3 blocks per SM 277).
+// Three-level ranks (n > 24) use the "both" classes alone.
+constexpr int kU1PairBlocks = 4, kPairUnroll = 6;  // resident blocks per SM; groups in flight
+template <typename R> __device__ __forceinline__ R pair_value(uint4 r);
+template <> __device__ __forceinline__ double pair_value<double>(uint4 r) {
+    return __hiloint2double(static_cast<int>(r.w), static_cast<int>(r.z));
+}
+template <> __device__ __forceinline__ float pair_value<float>(uint4 r) { return __uint_as_float(r.z); }
+
+template <typename R, int RK, bool DIAG>
+__global__ void __launch_bounds__(kU1Threads, kU1PairBlocks)
+    k_u1_pairs(U1Dev p, U1Apply a, const typename Cplx<R>::T *__restrict__ x, typename Cplx<R>::T *__restrict__ y,
+               uint64_t row0, uint64_t row1) {
+    using C = typename Cplx<R>::T;
+    constexpr int U = kPairUnroll;
+    extern __shared__ __align__(16) unsigned char sm[];
+    const uint4 *rec = reinterpret_cast<const uint4 *>(sm);
+    const uint32_t npairs = a.pair_seg[6];
+    uint32_t *tab = reinterpret_cast<uint32_t *>(sm + 16ull * npairs);
+    copy16(sm, sizeof(R) == 8 ? a.pairs : a.pairsf, 16ull * npairs);
+    copy16(reinterpret_cast<unsigned char *>(tab), a.ftab, a.ftab_bytes);
+    __syncthreads();
+    const uint32_t *basis = static_cast<const uint32_t *>(p.basis);
+    const uint64_t stride = static_cast<uint64_t>(gridDim.x) * blockDim.x;
+    for (uint64_t i = row0 + static_cast<uint64_t>(blockIdx.x) * blockDim.x + threadIdx.x; i < row1; i += stride) {
+        const uint32_t b = basis[i];
+        // the row's own halves of the rank
+        const uint32_t high = RK == 2 ? tab[a.h_off + (b >> a.rL)] : 0u;
+        const uint32_t low = RK == 2 ? static_cast<uint32_t>(i) - high : 0u;
+        R ar = 0, ai = 0, cr = 0, ci = 0;
+        if (DIAG) {
+            const double2 d = a.diag[i];
+            const R dr = static_cast<R>(d.x), di = static_cast<R>(d.y);
+            if (dr != R(0) || di != R(0)) {
+                const C xv = x[i];
+                ar = dr * xv.x - di * xv.y;
+                ai = dr * xv.y + di * xv.x;
+            }
+        }
+        auto walk = [&](auto where, auto signs, uint32_t g0, uint32_t g1) {
+            constexpr int WHERE = decltype(where)::value;  // 0 low half, 1 high half, 2 both
+            constexpr bool SIGNED = decltype(signs)::value;
+            for (uint32_t g = g0; g < g1; g += U) {
+                C xv[U];
+                R v[U];
+#pragma unroll
+                for (int u = 0; u < U; ++u) {
+                    const uint4 r = rec[g + u];
+                    const uint32_t t = b & r.x, src = b ^ r.x;
+                    uint32_t j;
+                    if constexpr (RK == 2 && WHERE == 0)
+                        j = high + tab[a.l_off + (src & a.lmask)];
+                    else if constexpr (RK == 2 && WHERE == 1)
+                        j = low + tab[a.h_off + (src >> a.rL)];
+                    else
+                        j = static_cast<uint32_t>(rank_any<RK, uint32_t, uint32_t>(src, tab, p, a));
+                    xv[u] = C{};
+                    if (t != 0u && t != r.x) xv[u] = x[j];
+                    v[u] = pair_value<R>(r);
+                    if (SIGNED && (__popc(r.y & b) & 1)) v[u] = -v[u];
+                }
+#pragma unroll
+                for (int u = 0; u < U; ++u) {
+                    if constexpr (sizeof(R) == 8) {
+                        ar = fma(v[u], xv[u].x, ar);
+                        ai = fma(v[u], xv[u].y, ai);
+                    } else {
+                        cmac<R, C>(ar, ai, cr, ci, v[u], R(0), xv[u]);
+                    }
+                }
+            }
+        };
+        using std::integral_constant;
+        if constexpr (RK == 2) {
+            walk(integral_constant<int, 0>{}, integral_constant<bool, false>{}, a.pair_seg[0], a.pair_seg[1]);
+            walk(integral_constant<int, 1>{}, integral_constant<bool, false>{}, a.pair_seg[1], a.pair_seg[2]);
+        }
+        walk(integral_constant<int, 2>{}, integral_constant<bool, false>{}, a.pair_seg[2], a.pair_seg[3]);
+        if constexpr (RK == 2) {
+            walk(integral_constant<int, 0>{}, integral_constant<bool, true>{}, a.pair_seg[3], a.pair_seg[4]);
+            walk(integral_constant<int, 1>{}, integral_constant<bool, true>{}, a.pair_seg[4], a.pair_seg[5]);
+        }
+        walk(integral_constant<int, 2>{}, integral_constant<bool, true>{}, a.pair_seg[5], a.pair_seg[6]);
         C out;
         out.x = ar;
         out.y = ai;
@@ -984,9 +1090,31 @@ int launch_apply_v(const tcp_u1_plan *p, const void *x, void *y, cudaStream_t s,
     return e == cudaSuccess ? TCP_OK : cuda_fail(e, "sector MVP kernel launch");
 }
 
+template <typename R, int RK, bool DIAG>
+int launch_pairs_v(const tcp_u1_plan *p, const void *x, void *y, cudaStream_t s, uint64_t row0, uint64_t row1) {
+    using C = typename Cplx<R>::T;
+    auto kern = k_u1_pairs<R, RK, DIAG>;
+    const size_t smem = 16ull * p->app.pair_seg[6] + p->app.ftab_bytes;
+    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));
+    if (e != cudaSuccess) return cuda_fail(e, "cudaFuncSetAttribute");
+    int per_sm = 0;
+    e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, kU1Threads, smem);
+    if (e != cudaSuccess) return cuda_fail(e, "cudaOccupancyMaxActiveBlocksPerMultiprocessor");
+    // one wave of resident CTAs: each CTA stages the tables once
+    const int grid = std::min<int>(grid_for(row1 - row0), std::max(per_sm, 1) * std::max(g_sms, 1));
+    kern<<<grid, kU1Threads, smem, s>>>(p->dev, p->app, static_cast<const C *>(x), static_cast<C *>(y), row0, row1);
+    e = cudaGetLastError();
+    return e == cudaSuccess ? TCP_OK : cuda_fail(e, "sector MVP kernel launch");
+}
+
 template <typename R, typename ST, typename IT, int RK>
 int launch_apply_t(const tcp_u1_plan *p, const void *x, void *y, cudaStream_t s, uint64_t r0, uint64_t r1) {
     const bool diag = p->app.diag != nullptr;
+    if constexpr (RK != 0) {
+        if (p->app.pairs) {
+            return diag ? launch_pairs_v<R, RK, true>(p, x, y, s, r0, r1) : launch_pairs_v<R, RK, false>(p, x, y, s, r0, r1);
+        }
+    }
     if (p->smem) {
         return diag ? launch_apply_v<R, ST, IT, RK, true, true>(p, x, y, s, r0, r1)
                     : launch_apply_v<R, ST, IT, RK, true, false>(p, x, y, s, r0, r1);
@@ -1252,6 +1380,36 @@ int upload(tcp_u1_plan *p) {
         ftab.insert(ftab.end(), Lr.begin(), Lr.end());
         fast.ftab_bytes = 4 * ftab.size();
     }
+    // Pair view: every group a real constant on two qubits, none general.
+    std::vector<uint32_t> pairs, pairsf;
+    uint32_t pair_seg[7] = {};
+    bool pairs_only = p->basis32 && NC == 0;
+    for (const auto *seg : {&segA, &segB})
+        for (const SegGroup &sg : *seg) pairs_only = pairs_only && (sg.x == 0 || (sg.half == 1 && sg.ci == 0.0));
+    if (pairs_only) {
+        for (int q = 0; q < 6; ++q) {
+            for (const SegGroup &sg : q < 3 ? segA : segB) {
+                if (sg.x == 0) continue;  // padding
+                const uint32_t sx = static_cast<uint32_t>(sg.x);
+                const bool in_low = (sx & ~fast.lmask) == 0, in_high = (sx & fast.lmask) == 0;
+                const int where = fast.rk != 2 ? 2 : (in_low ? 0 : (in_high ? 1 : 2));
+                if (where != q % 3) continue;
+                uint32_t w[2];
+                std::memcpy(w, &sg.cr, 8);
+                const float f = static_cast<float>(sg.cr);
+                uint32_t fw;
+                std::memcpy(&fw, &f, 4);
+                const uint32_t zo = static_cast<uint32_t>(sg.zout);
+                pairs.insert(pairs.end(), {sx, zo, w[0], w[1]});
+                pairsf.insert(pairsf.end(), {sx, zo, fw, 0u});
+            }
+            while ((pairs.size() / 4) % kPairUnroll) {  // x = 0: never live
+                pairs.insert(pairs.end(), 4, 0u);
+                pairsf.insert(pairsf.end(), 4, 0u);
+            }
+            pair_seg[q + 1] = static_cast<uint32_t>(pairs.size() / 4);
+        }
+    }
     Piece pieces[] = {
         {choose.data(), choose.size() * 8, 0},
         {p->index32 ? static_cast<const void *>(tab32.data()) : tab.data(), p->tab_bytes, 0},
@@ -1272,6 +1430,8 @@ int upload(tcp_u1_plan *p) {
         {awf.data(), 4ull * awf.size(), 0},
         {nullptr, has_diag ? 16 * p->dim : 0, 0},  // diagonal, evaluated on the device
         {ftab.data(), 4ull * ftab.size(), 0},
+        {pairs.data(), 4ull * pairs.size(), 0},
+        {pairsf.data(), 4ull * pairsf.size(), 0},
     };
     size_t off = 0;
     for (auto &pc : pieces) {
@@ -1355,6 +1515,11 @@ int upload(tcp_u1_plan *p) {
     p->smem_c128 = u1_apply_layout(apply_tab, NA, NB, NC, TA, ssz, 16).total;
     p->smem_c64 = u1_apply_layout(apply_tab, NA, NB, NC, TA, ssz, 8).total;
     p->smem = p->smem_c128 <= kU1SmemMax;
+    if (pairs_only && 4 * pairs.size() + ap.ftab_bytes <= kU1SmemMax) {
+        ap.pairs = reinterpret_cast<const uint4 *>(base + pieces[19].off);
+        ap.pairsf = reinterpret_cast<const uint4 *>(base + pieces[20].off);
+        std::copy(pair_seg, pair_seg + 7, ap.pair_seg);
+    }
     return TCP_OK;
 }
 
