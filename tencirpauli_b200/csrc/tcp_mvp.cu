@@ -1114,7 +1114,7 @@ int apply_host(const tcp_mvp_plan *plan, const R *state, uint64_t state_len, R *
     }
     HostCopies copies;
     int status = TCP_OK;
-    const bool large = bytes >= 2 * tcp::kStageSlotBytes;
+    const bool large = bytes >= tcp::kStageMinBytes;
     copies.stage_in = large && !page_locked(state);
     copies.stage_out = large && !page_locked(result);
     if (copies.stage_in || copies.stage_out) {
