@@ -505,34 +505,14 @@ class NativeMvpPlan:
         stream on the plan's device).  ``accumulate`` adds H x to y
         (``tcp_mvp_apply_add_device``) instead of overwriting it.
         """
-        import torch
-
-        if not (isinstance(x, torch.Tensor) and isinstance(y, torch.Tensor)):
-            raise TypeError("apply_device needs torch tensors")
-        if x.device.type != "cuda" or y.device.type != "cuda":
-            raise ValueError("apply_device needs CUDA tensors")
-        if x.dtype != y.dtype or x.dtype not in (torch.complex128, torch.complex64):
-            raise TypeError("apply_device tensors must both be complex128 or complex64")
-        if x.shape != y.shape or x.ndim not in (1, 2) or x.shape[-1] != self.dimension:
-            raise ValueError(f"apply_device tensors must have shape ({self.dimension},) or (nrhs, {self.dimension})")
-        if not (x.is_contiguous() and y.is_contiguous()):
-            raise ValueError("apply_device tensors must be contiguous")
-        nrhs = 1 if x.ndim == 1 else int(x.shape[0])
-        if stream is None:
-            stream = torch.cuda.current_stream(x.device)
-        handle = stream.cuda_stream if hasattr(stream, "cuda_stream") else int(stream)
-        dtype = TCP_DTYPE_C128 if x.dtype == torch.complex128 else TCP_DTYPE_C64
+        dimension = self.dimension
+        nrhs, dtype = _check_device_vectors(x, y, dimension)
         entry = self._lib.tcp_mvp_apply_add_device if accumulate else self._lib.tcp_mvp_apply_into_device
         status = entry(
-            self._handle,
-            ctypes.c_void_p(x.data_ptr()),
-            ctypes.c_void_p(y.data_ptr()),
-            self.dimension,
-            nrhs,
-            dtype,
-            ctypes.c_void_p(handle),
+            self._handle, x.data_ptr(), y.data_ptr(), dimension, nrhs, dtype, _stream_handle(stream, x.device)
         )
-        raise_for_status(status)
+        if status != TCP_OK:
+            raise_for_status(status)
 
     def diagonal_device(self, out: Any, stream: Any = None) -> None:
         """Write H_ii (complex128, the x_mask == 0 group) into a CUDA tensor."""
@@ -666,11 +646,43 @@ def number_commutator(nqubits: int, x_words: np.ndarray, z_words: np.ndarray, co
 
 
 def _stream_handle(stream: Any, device: Any) -> int:
-    import torch
-
+    """Raw handle of ``stream`` (None: torch's current stream on ``device``)."""
     if stream is None:
+        import torch
+
+        # the handle itself, without a Stream object around it (1 us per call)
+        raw = getattr(torch._C, "_cuda_getCurrentRawStream", None)
+        if raw is not None and device.index is not None:
+            return raw(device.index)
         stream = torch.cuda.current_stream(device)
     return stream.cuda_stream if hasattr(stream, "cuda_stream") else int(stream)
+
+
+def _check_device_vectors(x: Any, y: Any, dimension: int) -> Tuple[int, int]:
+    """(vectors, dtype code) of the buffers of a device apply.  A small apply is
+    bound by this Python path, so every attribute is read once."""
+    import torch
+
+    if not (isinstance(x, torch.Tensor) and isinstance(y, torch.Tensor)):
+        raise TypeError("apply_device needs torch tensors")
+    if not (x.is_cuda and y.is_cuda):
+        raise ValueError("apply_device needs CUDA tensors")
+    dtype = x.dtype
+    if dtype == torch.complex128:
+        code = TCP_DTYPE_C128
+    elif dtype == torch.complex64:
+        code = TCP_DTYPE_C64
+    else:
+        code = None
+    if code is None or y.dtype != dtype:
+        raise TypeError("apply_device tensors must both be complex128 or complex64")
+    shape = x.shape
+    ndim = len(shape)
+    if y.shape != shape or ndim not in (1, 2) or shape[-1] != dimension:
+        raise ValueError(f"apply_device tensors must have shape ({dimension},) or (nrhs, {dimension})")
+    if not (x.is_contiguous() and y.is_contiguous()):
+        raise ValueError("apply_device tensors must be contiguous")
+    return (1 if ndim == 1 else int(shape[0])), code
 
 
 class NativeU1Plan:
@@ -801,30 +813,13 @@ class NativeU1Plan:
 
     def apply_device(self, x: Any, y: Any, stream: Any = None) -> None:
         """Apply to torch CUDA tensors of shape (dim,) or (nrhs, dim)."""
-        import torch
-
-        if not (isinstance(x, torch.Tensor) and isinstance(y, torch.Tensor)):
-            raise TypeError("apply_device needs torch tensors")
-        if x.device.type != "cuda" or y.device.type != "cuda":
-            raise ValueError("apply_device needs CUDA tensors")
-        if x.dtype != y.dtype or x.dtype not in (torch.complex128, torch.complex64):
-            raise TypeError("apply_device tensors must both be complex128 or complex64")
-        if x.shape != y.shape or x.ndim not in (1, 2) or x.shape[-1] != self.dimension:
-            raise ValueError(f"apply_device tensors must have shape ({self.dimension},) or (nrhs, {self.dimension})")
-        if not (x.is_contiguous() and y.is_contiguous()):
-            raise ValueError("apply_device tensors must be contiguous")
-        nrhs = 1 if x.ndim == 1 else int(x.shape[0])
-        dtype = TCP_DTYPE_C128 if x.dtype == torch.complex128 else TCP_DTYPE_C64
+        dimension = self.dimension
+        nrhs, dtype = _check_device_vectors(x, y, dimension)
         status = self._lib.tcp_u1_apply_into_device(
-            self._handle,
-            ctypes.c_void_p(x.data_ptr()),
-            ctypes.c_void_p(y.data_ptr()),
-            self.dimension,
-            nrhs,
-            dtype,
-            ctypes.c_void_p(_stream_handle(stream, x.device)),
+            self._handle, x.data_ptr(), y.data_ptr(), dimension, nrhs, dtype, _stream_handle(stream, x.device)
         )
-        raise_for_status(status)
+        if status != TCP_OK:
+            raise_for_status(status)
 
     def diagonal_device(self, out: Any, stream: Any = None) -> None:
         import torch

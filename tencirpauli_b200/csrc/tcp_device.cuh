@@ -62,6 +62,8 @@ struct DevSchedule {
     const double2 *t_w;
     const float2 *t_wf;
     uint32_t ngroups;
+    uint32_t nterms;
+    const uint32_t *t_masks;  // n <= 11: x mask | z mask << 16 of each term (k_small)
 };
 
 // Step range [b0, b1) of host-path pass `pass` = p | log2(span) << 4 for

@@ -238,10 +238,10 @@ __global__ void __launch_bounds__(kThreads, 1)
 //    warp's chain of record load, sign, branch and multiply-adds is, with four
 //    warps per scheduler to hide it.  So the work per row counts: D is summed
 //    once per run and thread instead of multiplying every term into every row
-//    (2,000 random words on 28 qubits, complex128: 210 ms before, 190 now;
-//    Jordan-Wigner operator on 20 qubits: 30.7 before, 6.7 ms now), and 16 rows
+//    (2,000 random words on 28 qubits, complex128: 210 ms before, 169 now;
+//    Jordan-Wigner operator on 20 qubits: 30.7 before, 6.4 ms now), and 16 rows
 //    per thread halve the record walks per row (complex64, 26 qubits: 43.3 ms
-//    before, 38.4 with 8 rows, 26.3 with 16).  16 rows of complex64 with their
+//    before, 38.4 with 8 rows, 24.5 with 16).  16 rows of complex64 with their
 //    Kahan sums would need 128 registers beside the 32 of the loaded values;
 //    the Kahan sums, touched every kRingFoldRuns runs only, live in tensor
 //    memory (64 columns per warp), which this kernel otherwise has no use for.
@@ -496,6 +496,83 @@ __global__ void k_rowwise(DevSchedule s, const typename Cx<R>::T *__restrict__ x
     }
 }
 
+// States smaller than one ring tile (n < 12): S threads per row.  The state and
+// kSmallTerms terms at a time (x and z masks in one word, weight) are staged in
+// shared memory with one round of coalesced loads, and the S threads of a row
+// take the terms in turn and add up in FP64 by a fixed butterfly.  Such a call is
+// all latency: the row kernel's chain of dependent global loads per term took
+// 8.2 us on the device for a 10-qubit lattice, this takes 2.4.
+constexpr int kSmallThreads = 256;
+constexpr uint32_t kSmallTerms = 512;  // with 2^11 complex128: 42 KiB of static shared memory
+constexpr uint32_t kSmallMaxQubits = kTileBitsC128 - 1;  // masks below 16 bits
+
+template <typename R> struct SmallAcc;
+template <> struct SmallAcc<double> {
+    double re = 0.0, im = 0.0;
+    __device__ __forceinline__ void add(double2 w, double2 v) {
+        re = fma(w.x, v.x, fma(-w.y, v.y, re));
+        im = fma(w.x, v.y, fma(w.y, v.x, im));
+    }
+    __device__ __forceinline__ double2 sum() const { return make_double2(re, im); }
+};
+template <> struct SmallAcc<float> {  // FP32 products, Kahan-compensated sums
+    float re = 0.f, im = 0.f, cre = 0.f, cim = 0.f;
+    __device__ __forceinline__ void add(float2 w, float2 v) {
+        Acc<float>::kahan(re, cre, __fmaf_rn(w.x, v.x, -__fmul_rn(w.y, v.y)));
+        Acc<float>::kahan(im, cim, __fmaf_rn(w.x, v.y, __fmul_rn(w.y, v.x)));
+    }
+    __device__ __forceinline__ double2 sum() const {
+        return make_double2(static_cast<double>(re) - static_cast<double>(cre),
+                            static_cast<double>(im) - static_cast<double>(cim));
+    }
+};
+
+template <typename R, int S>
+__global__ void __launch_bounds__(kSmallThreads)
+    k_small(const uint32_t *__restrict__ masks, const typename Cx<R>::T *__restrict__ weights, uint32_t terms,
+            const typename Cx<R>::T *__restrict__ x, typename Cx<R>::T *__restrict__ y, uint32_t dim, uint64_t stride,
+            uint32_t accumulate) {
+    using C = typename Cx<R>::T;
+    __shared__ C xs[1u << kSmallMaxQubits], ws[kSmallTerms];
+    __shared__ uint32_t ms[kSmallTerms];
+    x += blockIdx.y * stride;
+    y += blockIdx.y * stride;
+    const uint32_t tid = threadIdx.x, sub = tid % S;
+    const uint32_t row = blockIdx.x * (kSmallThreads / S) + tid / S;
+    for (uint32_t i = tid; i < dim; i += kSmallThreads) xs[i] = x[i];
+    SmallAcc<R> acc;
+    for (uint32_t t0 = 0; t0 < terms; t0 += kSmallTerms) {
+        const uint32_t count = min(terms - t0, kSmallTerms);
+        if (t0) __syncthreads();
+        for (uint32_t t = tid; t < count; t += kSmallThreads) {
+            ws[t] = __ldg(&weights[t0 + t]);
+            ms[t] = __ldg(&masks[t0 + t]);
+        }
+        __syncthreads();
+        if (row < dim) {
+            for (uint32_t t = sub; t < count; t += S) {
+                const uint32_t m = ms[t], c = row ^ (m & 0xffffu);
+                const uint32_t odd = __popc((m >> 16) & c) & 1u;
+                const C w = ws[t];
+                acc.add(C{flip_by(w.x, odd), flip_by(w.y, odd)}, xs[c]);
+            }
+        }
+    }
+    double2 v = acc.sum();
+#pragma unroll
+    for (int off = S / 2; off > 0; off >>= 1) {
+        v.x += __shfl_xor_sync(0xffffffffu, v.x, off);
+        v.y += __shfl_xor_sync(0xffffffffu, v.y, off);
+    }
+    if (row < dim && sub == 0u) {
+        if (accumulate) {
+            v.x += static_cast<double>(y[row].x);
+            v.y += static_cast<double>(y[row].y);
+        }
+        y[row] = C{static_cast<R>(v.x), static_cast<R>(v.y)};
+    }
+}
+
 // Eager transition count: nonzero D_m[c] over all groups m and columns c, with
 // D summed in canonical term order exactly as hamiltonian.rs:125-133.
 __global__ void k_transitions(DevSchedule s, uint32_t ngroups, uint64_t dim, unsigned long long *count) {
@@ -636,6 +713,7 @@ int upload(tcp_mvp_plan *p) {
         const void **dst;
     };
     std::vector<Piece> pieces;
+    std::vector<uint32_t> small_masks;
     auto add = [&](const void *src, size_t bytes, const void **dst) { pieces.push_back({src, bytes, dst}); };
     {
         tcp::DeviceSchedule *ds = &p->sched;
@@ -648,6 +726,14 @@ int upload(tcp_mvp_plan *p) {
         add(h.t_z.data(), h.t_z.size() * 8, reinterpret_cast<const void **>(&ds->dev.t_z));
         add(h.t_w.data(), h.t_w.size() * 8, reinterpret_cast<const void **>(&ds->dev.t_w));
         add(h.t_wf.data(), h.t_wf.size() * 4, reinterpret_cast<const void **>(&ds->dev.t_wf));
+        if (p->nqubits <= kSmallMaxQubits) {
+            small_masks.reserve(h.t_z.size());
+            for (size_t g = 0; g < h.g_mask.size(); ++g)
+                for (uint32_t t = h.g_tbeg[g]; t < h.g_tbeg[g + 1]; ++t)
+                    small_masks.push_back(static_cast<uint32_t>(h.g_mask[g]) | static_cast<uint32_t>(h.t_z[t]) << 16);
+            add(small_masks.data(), small_masks.size() * 4, reinterpret_cast<const void **>(&ds->dev.t_masks));
+        }
+        ds->dev.nterms = static_cast<uint32_t>(h.t_z.size());
         ds->dev.nsteps = static_cast<uint32_t>(h.step_info.size() / 4);
         ds->dev.tile_bits = h.tile_bits;
         std::vector<uint64_t> pattern;  // outer pattern d of every step
@@ -801,6 +887,28 @@ template <typename R> int ensure_smem_attrs(int device) {
     return TCP_OK;
 }
 
+// Small states: `nrhs` vectors `stride` apart.  32 threads per row from 64
+// terms on, below that 8 (a warp would be half idle).
+template <typename R>
+void launch_small(const tcp_mvp_plan *p, const void *x, void *y, cudaStream_t stream, bool accumulate, uint32_t nrhs) {
+    using C = typename Cx<R>::T;
+    const DevSchedule &d = p->sched.dev;
+    const auto dim = static_cast<uint32_t>(p->dim);
+    const C *weights;
+    if constexpr (sizeof(R) == 8) weights = d.t_w;
+    else weights = d.t_wf;
+    const auto *xc = static_cast<const C *>(x);
+    auto *yc = static_cast<C *>(y);
+    const uint32_t add = accumulate ? 1u : 0u;
+    if (d.nterms >= 64) {
+        const dim3 grid((dim + kSmallThreads / 32 - 1) / (kSmallThreads / 32), nrhs);
+        k_small<R, 32><<<grid, kSmallThreads, 0, stream>>>(d.t_masks, weights, d.nterms, xc, yc, dim, dim, add);
+    } else {
+        const dim3 grid((dim + kSmallThreads / 8 - 1) / (kSmallThreads / 8), nrhs);
+        k_small<R, 8><<<grid, kSmallThreads, 0, stream>>>(d.t_masks, weights, d.nterms, xc, yc, dim, dim, add);
+    }
+}
+
 // Apply on `stream`; the tiled kernels write output tiles [tile0, tile0 +
 // ntiles) (ntiles = 0: all of them).  pass >= 0 runs one source-part pass of
 // the host path, adding to y when `accumulate`.
@@ -836,6 +944,8 @@ int launch_one(const tcp_mvp_plan *p, const void *x, void *y, cudaStream_t strea
             k_tiled<LOGE, R, false><<<static_cast<unsigned>(tiles), kThreads, smem, stream>>>(
                 ds.dev, static_cast<const C *>(x), static_cast<C *>(y), p->d_err, tile0, 0u, accumulate ? 1u : 0u);
         }
+    } else if (p->nqubits <= kSmallMaxQubits) {
+        launch_small<R>(p, x, y, stream, accumulate, 1);
     } else {
         const int threads = 256;
         uint64_t blocks = (p->dim + threads - 1) / threads;
@@ -1383,6 +1493,14 @@ int apply_device(const tcp_mvp_plan *plan, const void *d_state, void *d_result, 
     // a block of vectors: one ring launch over tiles x vectors
     if (nrhs > 1 && nrhs <= 65535u && ring_ok(plan, d_state) && (reinterpret_cast<uintptr_t>(d_result) % 16) == 0)
         return tcp::launch_ring_rhs(plan, d_state, d_result, nrhs, dtype == TCP_DTYPE_C64, plan->d_err, s, accumulate);
+    if (plan->nqubits <= kSmallMaxQubits && nrhs <= 65535u) {
+        if (dtype == TCP_DTYPE_C128)
+            launch_small<double>(plan, d_state, d_result, s, accumulate, nrhs);
+        else
+            launch_small<float>(plan, d_state, d_result, s, accumulate, nrhs);
+        cudaError_t e = cudaGetLastError();
+        return e == cudaSuccess ? TCP_OK : cuda_fail(e, "MVP kernel launch");
+    }
     for (uint32_t v = 0; v < nrhs; ++v) {
         const void *x = static_cast<const unsigned char *>(d_state) + static_cast<size_t>(v) * len * elem;
         void *y = static_cast<unsigned char *>(d_result) + static_cast<size_t>(v) * len * elem;
@@ -1572,6 +1690,8 @@ extern "C" int tcp_mvp_apply_into_host_noalloc(const tcp_mvp_plan *plan, const d
         const size_t smem = tiled_smem_bytes<kLogRowsC128, double>();
         k_tiled<kLogRowsC128, double, false><<<static_cast<unsigned>(plan->dim >> S), kThreads, smem, s>>>(
             ds.dev, dx, dy, d_status, 0, 0u, 0u);
+    } else if (plan->nqubits <= kSmallMaxQubits) {
+        launch_small<double>(plan, dx, dy, s, false, 1);
     } else {
         const int threads = 256;
         const uint64_t blocks = (plan->dim + threads - 1) / threads;
