@@ -29,7 +29,12 @@ constexpr int kErrTimeout = 1;
 constexpr int kErrBounds = 2;  // TCP_DEBUG_BOUNDS builds: a block failed its bounds check
 
 // Ring view (k_ring; see tcp::RingSchedule): steps = 0 when the plan has no
-// schedule of this shape.  Pass ranges as in DevSchedule, over the ring steps.
+// schedule of this shape.
+// Source-part passes of the host path: steps [pass_begin[v], pass_begin[v + 1])
+// have outer patterns d whose top kPassBits bits equal v (steps are sorted by
+// d), so an output tile t reads source tiles t ^ d in part v ^ (t >>
+// pass_shift) of the kPassChunks equal parts of the state (pass_range).
+// pass_shift = kNoPasses when the state has fewer than kPassChunks tiles.
 struct RingView {
     const uint4 *info;              // 4 words per step, see tcp::RingSchedule::step_info
     const unsigned char *blocks128;  // blocks with FP64 weights
@@ -40,20 +45,6 @@ struct RingView {
 };
 
 struct DevSchedule {
-    // step view (tiled kernels); see tcp::Schedule
-    const uint4 *step_info;          // d lo, d hi, block offset / 16, ngroups | (bytes / 16) << 16
-    const unsigned char *blocks128;  // step blocks with FP64 weights
-    const unsigned char *blocks64;   // step blocks with FP32 weights
-    uint32_t nsteps;
-    uint32_t tile_bits;
-    // Source-part passes of the host path: steps [pass_begin[v],
-    // pass_begin[v + 1]) have outer patterns d whose top kPassBits bits equal
-    // v (steps are sorted by d), so an output tile t reads source tiles t ^ d
-    // in part v ^ (t >> pass_shift) of the kPassChunks equal parts of the
-    // state (pass_range).  pass_shift = kNoPasses when the state has fewer
-    // than kPassChunks tiles.
-    uint32_t pass_begin[kPassChunks + 1];
-    uint32_t pass_shift;
     RingView ring[tcp::kRingShapeCount];  // k_ring's schedules, one per shape
     // group view (row kernel, transition count, diagonal): unfolded weights
     const uint64_t *g_mask;

@@ -45,7 +45,7 @@ struct MatrixTerm {
     double w_im;
 };
 
-// Tile schedule for the tiled kernels.  The 2^n rows are cut into tiles of
+// Tile schedule for the batched kernel.  The 2^n rows are cut into tiles of
 // 2^tile_bits consecutive rows.  Every x-mask group m splits into an outer
 // pattern d = m >> tile_bits (which source tile feeds an output tile: the tile
 // index XOR d) and an inner mask m & (2^tile_bits - 1) (a permutation inside
@@ -67,7 +67,7 @@ struct Schedule {
     uint32_t tile_bits = 0;
     uint32_t log_threads = 0;
     uint64_t distinct_outer = 0;      // distinct outer patterns d
-    // step view (tiled kernels).  A step is one outer pattern d and a block of
+    // step view (k_batched).  A step is one outer pattern d and a block of
     // its groups and terms no larger than kBlockBytesMax; a pattern with more
     // data is split over several steps (the tile is loaded once per step).
     // step_info: 4 words per step: d (lo, hi), block offset / 16,
@@ -127,7 +127,8 @@ struct Schedule {
 // The word (kRing* below) names the run (a, imag, row signs to flip) and tells
 // where it ends, where a coset begins (the 8 source values are loaded then)
 // and, complex64, where the partial sums are folded into the compensated row
-// sums (a new coset follows a fold, so no loaded values live across it).  Records are 16-byte aligned and the next one is loaded while the
+// sums (in a schedule without complex128 blocks a new coset follows a fold, so
+// that the 16-row kernel holds no loaded values across it).  Records are 16-byte aligned and the next one is loaded while the
 // present one is applied, so a block leaves 16 bytes of its stage unused.
 constexpr uint32_t kRingImag = 1u << 4;       // bits 0..3: the register permutation a
 constexpr uint32_t kRingKindShift = 5;        // 0 single, 1 / 2 / 3: table of 4 / 8 / 16
@@ -184,8 +185,9 @@ enum : uint32_t { kKindReal = 0, kKindImag = 1, kKindComplex = 2 };
 // (group_matrix_terms, hamiltonian.rs:573-582); terms keep canonical order
 // inside a group so the per-group diagonal sum rounds exactly as the
 // reference's eager diagonal (hamiltonian.rs:125-133).
+// `blocks` = false leaves the step blocks out (step_info still counts them).
 Schedule build_schedule(const std::vector<MatrixTerm> &terms, uint32_t nqubits, uint32_t tile_bits,
-                        uint32_t log_threads);
+                        uint32_t log_threads, bool blocks = true);
 
 // Compile packed words into matrix terms (pauli_action.rs:24-88).
 int compile_terms(uint32_t nqubits, uint64_t count, uint32_t word_count, const uint64_t *x_words,

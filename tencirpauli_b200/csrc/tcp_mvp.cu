@@ -1,17 +1,17 @@
 // libtcpmvp.so -- sm_100a kernels and the C ABI of the matrix-free Pauli MVP.
 //
 // Kernels (all hand-written for sm_100a):
-//   k_tiled     tile-staged grouped MVP.  One CTA owns an output tile of
-//               2^S consecutive rows and keeps its accumulators in registers;
-//               for every outer pattern d ("step") the source tile
-//               (tile ^ d) is copied into shared memory by the TMA bulk-copy
-//               engine (cp.async.bulk + mbarrier, double-buffered), and every
-//               x-mask group of that step is applied from shared memory:
+//   k_ring      the tiled MVP.  One CTA owns an output tile of consecutive rows
+//               and keeps its sums in registers; for every outer pattern d
+//               ("step") the source tile (tile ^ d) is copied into shared
+//               memory by the TMA bulk-copy engine, and every x-mask group of
+//               that step is applied from there:
 //               D_m(c) = sum_{k in m} w_k (-1)^{popcount(z_k & c)} evaluated
 //               at the source column c = r ^ m, then y[r] += D_m(c) x[c].
 //               FP64 (complex128) and FP32-with-Kahan (complex64) variants.
-//   k_rowwise   one thread per row, direct gathers; for states smaller than
-//               one tile and for buffers the bulk-copy engine cannot address.
+//   k_small     states below one tile (n < 12), staged whole in shared memory.
+//   k_rowwise   one thread per row, direct gathers; for buffers the bulk-copy
+//               engine cannot address and plans without a ring schedule.
 //   k_transitions / k_diagonal   eager transition count and H_ii extraction.
 //
 // Reference semantics (paths inside the reference project):
@@ -42,189 +42,6 @@ using namespace tcpdev;
 namespace {
 
 // --------------------------------- kernels ---------------------------------
-// One term applied to the thread's E rows.  `rec` is the term record's first
-// 16 bytes (zlo | (pattern | kind << 24) << 32, zt); `w` its weight with the
-// per-step and per-group signs already folded in.  The remaining sign,
-// parity(zlo & tid) ^ parity(zt & tile), is one POPC of an XOR (the parity of
-// a XOR equals the XOR of the parities).
-template <int JH, int LOGE, typename R>
-__device__ __forceinline__ void apply_term(ulonglong2 rec, typename Cx<R>::T w, uint32_t tid, uint64_t tile,
-                                           const typename Cx<R>::T (&xv)[1 << LOGE], Acc<R> (&acc)[1 << LOGE]) {
-    constexpr int E = 1 << LOGE;
-    constexpr uint32_t kPatMask = (1u << E) - 1u;
-    const uint32_t lo = static_cast<uint32_t>(rec.x);
-    const uint32_t hi = static_cast<uint32_t>(rec.x >> 32);
-    const uint64_t zt_tile = rec.y & tile;
-    const uint32_t base =
-        __popc((lo & tid) ^ static_cast<uint32_t>(zt_tile) ^ static_cast<uint32_t>(zt_tile >> 32)) & 1u;
-    const uint32_t pattern = hi & kPatMask;
-    const uint32_t kind = hi >> 24;
-    if (pattern == 0u) {
-        const R wr = flip_by(w.x, base), wi = flip_by(w.y, base);
-        if (kind == tcp::kKindReal) {
-#pragma unroll
-            for (int jj = 0; jj < E; ++jj) acc[jj ^ JH].add_real(wr, xv[jj]);
-        } else if (kind == tcp::kKindImag) {
-#pragma unroll
-            for (int jj = 0; jj < E; ++jj) acc[jj ^ JH].add_imag(wi, xv[jj]);
-        } else {
-#pragma unroll
-            for (int jj = 0; jj < E; ++jj) acc[jj ^ JH].add_complex(wr, wi, xv[jj]);
-        }
-    } else {
-        const uint32_t pat = (pattern ^ (0u - base)) & kPatMask;  // sign bit of every source jj
-        if (kind == tcp::kKindReal) {
-#pragma unroll
-            for (int jj = 0; jj < E; ++jj) acc[jj ^ JH].add_real(flip_if(w.x, pat, jj), xv[jj]);
-        } else if (kind == tcp::kKindImag) {
-#pragma unroll
-            for (int jj = 0; jj < E; ++jj) acc[jj ^ JH].add_imag(flip_if(w.y, pat, jj), xv[jj]);
-        } else {
-#pragma unroll
-            for (int jj = 0; jj < E; ++jj)
-                acc[jj ^ JH].add_complex(flip_if(w.x, pat, jj), flip_if(w.y, pat, jj), xv[jj]);
-        }
-    }
-}
-
-// Terms of one x-mask group applied to the thread's E rows.  JH is a
-// compile-time row permutation between the loaded values and the rows; the
-// tiled kernel loads its values in row order already (JH = 0).
-// Term records come from the step block in shared memory; a term whose z mask
-// has no bit among the thread's row bits (pattern 0) has one sign for all E
-// rows, otherwise the sign of source jj is bit jj of the pattern.
-template <int JH, int LOGE, typename R>
-__device__ __forceinline__ void apply_group(const unsigned char *__restrict__ trm, uint32_t tb, uint32_t te,
-                                            uint32_t tid, uint64_t tile, const typename Cx<R>::T (&xv)[1 << LOGE],
-                                            Acc<R> (&acc)[1 << LOGE]) {
-    for (uint32_t t = tb; t < te; ++t) {
-        const unsigned char *r0 = trm + t * tcp::kTermRecBytes;
-        apply_term<JH, LOGE, R>(*reinterpret_cast<const ulonglong2 *>(r0), record_weight<R>(r0), tid, tile, xv, acc);
-    }
-}
-
-// Source values of one group for the thread, in row order: row j of the
-// thread (tile row tid + j * T) reads source tile row (tid ^ m_lo) +
-// (j ^ jh) * T, where m_lo and jh are the group's inner-mask bits at and
-// above the thread index.
-template <int LOGE, typename C>
-__device__ __forceinline__ void load_group(const C *__restrict__ xs, uint32_t tid, uint32_t m, C (&xv)[1 << LOGE]) {
-    const C *src = xs + (tid ^ (m & (kThreads - 1)));
-    const uint32_t jh = m >> kLogThreads;
-#pragma unroll
-    for (int j = 0; j < (1 << LOGE); ++j) xv[j] = src[(static_cast<uint32_t>(j) ^ jh) << kLogThreads];
-}
-
-template <typename R> __device__ __forceinline__ const unsigned char *step_blocks(const DevSchedule &s);
-template <> __device__ __forceinline__ const unsigned char *step_blocks<double>(const DevSchedule &s) {
-    return s.blocks128;
-}
-template <> __device__ __forceinline__ const unsigned char *step_blocks<float>(const DevSchedule &s) {
-    return s.blocks64;
-}
-
-// Issue the bulk copies of one step (source tile + step block) on one mbarrier.
-template <typename C, uint32_t S>
-__device__ __forceinline__ void issue_step(const uint4 info, uint64_t tile, const C *__restrict__ x,
-                                           const unsigned char *__restrict__ blocks, C *tile_dst,
-                                           unsigned char *blk_dst, uint64_t *bar) {
-    constexpr uint32_t BYTES = (1u << S) * sizeof(C);
-    const uint64_t d = static_cast<uint64_t>(info.x) | (static_cast<uint64_t>(info.y) << 32);
-    const uint32_t blk_bytes = (info.w >> 16) * 16u;
-    mbar_arrive_expect_tx(bar, BYTES + blk_bytes);
-    bulk_copy_g2s(tile_dst, x + ((tile ^ d) << S), BYTES, bar);
-    bulk_copy_g2s(blk_dst, blocks + static_cast<size_t>(info.z) * 16u, blk_bytes, bar);
-}
-
-// Tile-staged grouped MVP (see file header).  Grid: one CTA per output tile;
-// thread t owns rows t + j * kThreads of the tile.  Shared memory: two source
-// tiles and two step blocks (double buffering), refilled by the TMA engine.
-// PASSES = false runs every step and overwrites y.  PASSES = true runs pass
-// `pass` (0..kPassChunks-1): only the steps whose source tiles lie in part
-// `pass` of the state (see DevSchedule::pass_begin), adding to y when
-// `accumulate`.
-template <int LOGE, typename R, bool PASSES>
-__global__ void __launch_bounds__(kThreads, 1)
-    k_tiled(DevSchedule s, const typename Cx<R>::T *__restrict__ x, typename Cx<R>::T *__restrict__ y,
-            int *__restrict__ err, uint64_t tile0, uint32_t pass, uint32_t accumulate) {
-    using C = typename Cx<R>::T;
-    static_assert(LOGE == 3, "the group dispatch below covers 8 rows per thread");
-    constexpr int E = 1 << LOGE;
-    constexpr int S = kLogThreads + LOGE;
-    constexpr uint32_t TILE = 1u << S;
-    extern __shared__ __align__(128) unsigned char smem_raw[];
-    C *tiles = reinterpret_cast<C *>(smem_raw);
-    unsigned char *blks = smem_raw + 2 * TILE * sizeof(C);
-    __shared__ __align__(8) uint64_t bars[2];
-
-    const uint32_t tid = threadIdx.x;
-    const uint64_t tile = tile0 + blockIdx.x;
-    uint32_t step0 = 0, nsteps = s.nsteps;
-    if constexpr (PASSES) {
-        uint32_t b0, b1;
-        pass_range(s.pass_begin, s.pass_shift, tile, pass, b0, b1);
-        step0 = b0;
-        nsteps = b1 - b0;
-    }
-    const uint4 *steps = s.step_info + step0;
-    const unsigned char *blocks = step_blocks<R>(s);
-
-    if (tid == 0) {
-        mbar_init(&bars[0], 1);
-        mbar_init(&bars[1], 1);
-        fence_mbar_init();
-    }
-    __syncthreads();
-    if (tid == 0 && nsteps > 0) issue_step<C, S>(__ldg(&steps[0]), tile, x, blocks, tiles, blks, &bars[0]);
-
-    Acc<R> acc[E];
-    for (uint32_t st = 0; st < nsteps; ++st) {
-        const uint32_t b = st & 1u;
-        const uint4 info = __ldg(&steps[st]);
-        const bool ok = mbar_wait_bounded(&bars[b], (st >> 1) & 1u);
-        if (__syncthreads_or(!ok)) {
-            if (tid == 0) atomicOr(err, kErrTimeout);
-            return;
-        }
-        // Every thread has finished step st-1, so the other buffers are free.
-        if (tid == 0 && st + 1 < nsteps) {
-            fence_proxy_async_smem();
-            issue_step<C, S>(__ldg(&steps[st + 1]), tile, x, blocks, tiles + (b ^ 1u) * TILE,
-                             blks + (b ^ 1u) * tcp::kBlockBytesMax, &bars[b ^ 1u]);
-        }
-        const C *xs = tiles + b * TILE;
-        const unsigned char *blk = blks + b * tcp::kBlockBytesMax;
-        const uint32_t ng = info.w & 0xffffu;
-        const uint4 *grp = reinterpret_cast<const uint4 *>(blk);
-        const unsigned char *trm = blk + ng * tcp::kGroupRecBytes;
-        for (uint32_t g = 0; g < ng; ++g) {
-            const uint4 gr = grp[g];
-            C xv[E];
-            load_group<LOGE>(xs, tid, gr.x, xv);
-            apply_group<0, LOGE, R>(trm, gr.y, gr.z, tid, tile, xv, acc);
-            // FP32: fold the running group sum into the compensated row sum
-            // every kCompensateGroups groups and at the end of the step.
-            if (((g + 1) % kCompensateGroups) == 0u || g + 1 == ng) {
-#pragma unroll
-                for (int j = 0; j < E; ++j) acc[j].compensate();
-            }
-        }
-    }
-    C *yt = y + (tile << S);
-    if (accumulate) {
-#pragma unroll
-        for (int j = 0; j < E; ++j) {
-            C &out = yt[tid + (j << kLogThreads)];
-            const C v = acc[j].value();
-            out.x += v.x;
-            out.y += v.y;
-        }
-    } else {
-#pragma unroll
-        for (int j = 0; j < E; ++j) yt[tid + (j << kLogThreads)] = acc[j].value();
-    }
-}
-
 // ------------------------------- ring kernel --------------------------------
 // k_ring: the tiled MVP with a ring of source tiles.
 //  * Sixteen warps own the output tile's rows and keep their sums in
@@ -718,9 +535,6 @@ int upload(tcp_mvp_plan *p) {
     {
         tcp::DeviceSchedule *ds = &p->sched;
         tcp::Schedule &h = ds->host;
-        add(h.step_info.data(), h.step_info.size() * 4, reinterpret_cast<const void **>(&ds->dev.step_info));
-        add(h.blocks_c128.data(), h.blocks_c128.size(), reinterpret_cast<const void **>(&ds->dev.blocks128));
-        add(h.blocks_c64.data(), h.blocks_c64.size(), reinterpret_cast<const void **>(&ds->dev.blocks64));
         add(h.g_mask.data(), h.g_mask.size() * 8, reinterpret_cast<const void **>(&ds->dev.g_mask));
         add(h.g_tbeg.data(), h.g_tbeg.size() * 4, reinterpret_cast<const void **>(&ds->dev.g_tbeg));
         add(h.t_z.data(), h.t_z.size() * 8, reinterpret_cast<const void **>(&ds->dev.t_z));
@@ -734,12 +548,6 @@ int upload(tcp_mvp_plan *p) {
             add(small_masks.data(), small_masks.size() * 4, reinterpret_cast<const void **>(&ds->dev.t_masks));
         }
         ds->dev.nterms = static_cast<uint32_t>(h.t_z.size());
-        ds->dev.nsteps = static_cast<uint32_t>(h.step_info.size() / 4);
-        ds->dev.tile_bits = h.tile_bits;
-        std::vector<uint64_t> pattern;  // outer pattern d of every step
-        for (size_t i = 0; i < h.step_info.size(); i += 4)
-            pattern.push_back(h.step_info[i] | static_cast<uint64_t>(h.step_info[i + 1]) << 32);
-        set_passes(pattern, h.tile_bits, p->nqubits, ds->dev.pass_begin, &ds->dev.pass_shift);
         for (int shape = 0; shape < tcp::kRingShapeCount; ++shape) {
             tcp::RingSchedule &r = ds->ring[shape];
             RingView &v = ds->dev.ring[shape];
@@ -747,7 +555,7 @@ int upload(tcp_mvp_plan *p) {
             add(r.blocks_c128.data(), r.blocks_c128.size(), reinterpret_cast<const void **>(&v.blocks128));
             add(r.blocks_c64.data(), r.blocks_c64.size(), reinterpret_cast<const void **>(&v.blocks64));
             v.steps = static_cast<uint32_t>(r.step_info.size() / 4);
-            pattern.clear();
+            std::vector<uint64_t> pattern;  // outer pattern d of every step
             for (size_t i = 0; i < r.step_info.size(); i += 4) pattern.push_back(r.step_info[i]);
             set_passes(pattern, r.tile_bits, p->nqubits, v.pass_begin, &v.pass_shift);
         }
@@ -782,20 +590,6 @@ int upload(tcp_mvp_plan *p) {
 
 
 
-
-template <int LOGE, typename R> constexpr size_t tiled_smem_bytes() {
-    return 2 * (size_t(1) << (kLogThreads + LOGE)) * sizeof(typename Cx<R>::T) + 2 * size_t(tcp::kBlockBytesMax);
-}
-
-template <int LOGE, typename R> int set_smem_attr() {
-    constexpr size_t bytes = tiled_smem_bytes<LOGE, R>();
-    cudaError_t e = cudaFuncSetAttribute(k_tiled<LOGE, R, false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                         static_cast<int>(bytes));
-    if (e == cudaSuccess)
-        e = cudaFuncSetAttribute(k_tiled<LOGE, R, true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                 static_cast<int>(bytes));
-    return e == cudaSuccess ? TCP_OK : cuda_fail(e, "cudaFuncSetAttribute");
-}
 
 template <typename K> int opt_in_smem(K *kernel, size_t bytes) {
     cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(bytes));
@@ -851,33 +645,27 @@ void launch_ring(const tcp_mvp_plan *p, const void *x, void *y, int *err, cudaSt
         k_ring<R, SHAPE, false><<<grid, G::kThreads, G::kSmemBytes, stream>>>(v, xc, yc, err, tile0, 0u, add, 0ull);
 }
 
-// Number of output tiles of the tiled kernels (0 when the plan uses the row
-// kernel for these buffers).
+// Number of output tiles (0 when the plan does not run the ring kernel on
+// these buffers).
 template <typename R>
 uint64_t tiled_tiles(const tcp_mvp_plan *p, const void *x, const void *y) {
-    constexpr int LOGE = sizeof(R) == 8 ? kLogRowsC128 : kLogRowsC64;
-    const uint32_t S = kLogThreads + LOGE;
-    const bool aligned = (reinterpret_cast<uintptr_t>(x) % 16) == 0;
-    if (ring_ok(p, x)) return p->dim >> tcp::kRingShapes[ring_shape<R>(p, y, 1)].tile_bits;
-    return (p->nqubits >= S && p->sched.host.tile_bits == S && aligned) ? (p->dim >> S) : 0;
+    return ring_ok(p, x) ? p->dim >> tcp::kRingShapes[ring_shape<R>(p, y, 1)].tile_bits : 0;
 }
 
 // Whether the host path can split the state into kPassChunks parts for the
 // kernel that serves these buffers.
 template <typename R> bool has_passes(const tcp_mvp_plan *p, const void *x, const void *y) {
-    return (ring_ok(p, x) ? p->sched.dev.ring[ring_shape<R>(p, y, 1)].pass_shift : p->sched.dev.pass_shift) != kNoPasses;
+    return ring_ok(p, x) && p->sched.dev.ring[ring_shape<R>(p, y, 1)].pass_shift != kNoPasses;
 }
 
-// Per-device, once: the shared-memory opt-in of the tiled kernels.
+// Per-device, once: the shared-memory opt-in of the ring kernel.
 template <typename R> int ensure_smem_attrs(int device) {
     static std::mutex attr_mutex;
     static bool attr_done[64] = {};
     std::lock_guard<std::mutex> lock(attr_mutex);
     if (device < 0 || device >= 64) return fail(TCP_ERR_WRONG_DEVICE, "device ordinal out of range");
     if (!attr_done[device]) {
-        constexpr int LOGE = sizeof(R) == 8 ? kLogRowsC128 : kLogRowsC64;
-        int st = set_smem_attr<LOGE, R>();
-        if (st == TCP_OK) st = set_ring_smem_attr<R, 0>();
+        int st = set_ring_smem_attr<R, 0>();
         if constexpr (sizeof(R) == 4) {
             if (st == TCP_OK) st = set_ring_smem_attr<R, 1>();
         }
@@ -909,18 +697,13 @@ void launch_small(const tcp_mvp_plan *p, const void *x, void *y, cudaStream_t st
     }
 }
 
-// Apply on `stream`; the tiled kernels write output tiles [tile0, tile0 +
+// Apply on `stream`; the ring kernel writes output tiles [tile0, tile0 +
 // ntiles) (ntiles = 0: all of them).  pass >= 0 runs one source-part pass of
 // the host path, adding to y when `accumulate`.
 template <typename R>
 int launch_one(const tcp_mvp_plan *p, const void *x, void *y, cudaStream_t stream, uint64_t tile0 = 0,
                uint64_t ntiles = 0, int pass = -1, bool accumulate = false) {
     using C = typename Cx<R>::T;
-    constexpr bool is64 = sizeof(R) == 8;
-    constexpr int LOGE = is64 ? kLogRowsC128 : kLogRowsC64;
-    const tcp::DeviceSchedule &ds = p->sched;
-    const uint32_t S = kLogThreads + LOGE;
-    const bool aligned = (reinterpret_cast<uintptr_t>(x) % 16) == 0;
     if (ring_ok(p, x)) {
         int st = ensure_smem_attrs<R>(p->device);
         if (st != TCP_OK) return st;
@@ -931,19 +714,6 @@ int launch_one(const tcp_mvp_plan *p, const void *x, void *y, cudaStream_t strea
         } else if constexpr (sizeof(R) == 4) {
             launch_ring<R, 1>(p, x, y, p->d_err, stream, tile0, tiles, pass, accumulate, 1);
         }
-    } else if (p->nqubits >= S && ds.host.tile_bits == S && aligned) {
-        int st = ensure_smem_attrs<R>(p->device);
-        if (st != TCP_OK) return st;
-        const uint64_t tiles = ntiles ? ntiles : (p->dim >> S) - tile0;
-        const size_t smem = tiled_smem_bytes<LOGE, R>();
-        if (pass >= 0) {
-            k_tiled<LOGE, R, true><<<static_cast<unsigned>(tiles), kThreads, smem, stream>>>(
-                ds.dev, static_cast<const C *>(x), static_cast<C *>(y), p->d_err, tile0, static_cast<uint32_t>(pass),
-                accumulate ? 1u : 0u);
-        } else {
-            k_tiled<LOGE, R, false><<<static_cast<unsigned>(tiles), kThreads, smem, stream>>>(
-                ds.dev, static_cast<const C *>(x), static_cast<C *>(y), p->d_err, tile0, 0u, accumulate ? 1u : 0u);
-        }
     } else if (p->nqubits <= kSmallMaxQubits) {
         launch_small<R>(p, x, y, stream, accumulate, 1);
     } else {
@@ -951,7 +721,7 @@ int launch_one(const tcp_mvp_plan *p, const void *x, void *y, cudaStream_t strea
         uint64_t blocks = (p->dim + threads - 1) / threads;
         blocks = std::min<uint64_t>(blocks, 1u << 20);
         k_rowwise<R><<<static_cast<unsigned>(blocks), threads, 0, stream>>>(
-            ds.dev, static_cast<const C *>(x), static_cast<C *>(y), p->dim, accumulate ? 1u : 0u);
+            p->sched.dev, static_cast<const C *>(x), static_cast<C *>(y), p->dim, accumulate ? 1u : 0u);
     }
     cudaError_t e = cudaGetLastError();
     return e == cudaSuccess ? TCP_OK : cuda_fail(e, "MVP kernel launch");
@@ -1410,7 +1180,7 @@ extern "C" int tcp_mvp_plan_create(uint32_t nqubits, uint64_t term_count, uint32
     if (g_num_sms == 0) cudaDeviceGetAttribute(&g_num_sms, cudaDevAttrMultiProcessorCount, p->device);
     {
         tcp::Range range("tile schedules");
-        p->sched.host = tcp::build_schedule(p->terms, nqubits, kTileBitsC128, kLogThreads);
+        p->sched.host = tcp::build_schedule(p->terms, nqubits, kTileBitsC128, kLogThreads, false);
         p->sched.ring[0] = tcp::build_ring_schedule(p->terms, nqubits, tcp::kRingShapes[0]);
         p->sched.ring[1] = tcp::build_ring_schedule(p->terms, nqubits, tcp::kRingShapes[1], false);
     }
@@ -1682,20 +1452,14 @@ extern "C" int tcp_mvp_apply_into_host_noalloc(const tcp_mvp_plan *plan, const d
     if (e != cudaSuccess) return cuda_fail(e, "clearing the static scratch status");
     e = cudaMemcpyAsync(dx, state, bytes, cudaMemcpyHostToDevice, s);
     if (e != cudaSuccess) return cuda_fail(e, "H2D copy into the static scratch");
-    const tcp::DeviceSchedule &ds = plan->sched;
-    const uint32_t S = kTileBitsC128;
     if (ring_ok(plan, dx)) {
-        launch_ring<double, 0>(plan, dx, dy, d_status, s, 0, plan->dim >> S, -1, false, 1);
-    } else if (plan->nqubits >= S && ds.host.tile_bits == S) {
-        const size_t smem = tiled_smem_bytes<kLogRowsC128, double>();
-        k_tiled<kLogRowsC128, double, false><<<static_cast<unsigned>(plan->dim >> S), kThreads, smem, s>>>(
-            ds.dev, dx, dy, d_status, 0, 0u, 0u);
+        launch_ring<double, 0>(plan, dx, dy, d_status, s, 0, plan->dim >> kTileBitsC128, -1, false, 1);
     } else if (plan->nqubits <= kSmallMaxQubits) {
         launch_small<double>(plan, dx, dy, s, false, 1);
     } else {
         const int threads = 256;
         const uint64_t blocks = (plan->dim + threads - 1) / threads;
-        k_rowwise<double><<<static_cast<unsigned>(blocks), threads, 0, s>>>(ds.dev, dx, dy, plan->dim, 0u);
+        k_rowwise<double><<<static_cast<unsigned>(blocks), threads, 0, s>>>(plan->sched.dev, dx, dy, plan->dim, 0u);
     }
     e = cudaGetLastError();
     if (e != cudaSuccess) return cuda_fail(e, "MVP kernel launch");

@@ -118,7 +118,7 @@ template <typename T> void put(std::vector<uint8_t> &out, const T &v) {
 }  // namespace
 
 Schedule build_schedule(const std::vector<MatrixTerm> &terms, uint32_t nqubits, uint32_t tile_bits,
-                        uint32_t log_threads) {
+                        uint32_t log_threads, bool blocks) {
     Schedule s;
     s.tile_bits = std::min(tile_bits, nqubits);
     s.log_threads = std::min(log_threads, s.tile_bits);
@@ -162,6 +162,13 @@ Schedule build_schedule(const std::vector<MatrixTerm> &terms, uint32_t nqubits, 
     size_t pend_bytes = 0;
     auto flush = [&]() {
         if (pend.empty()) return;
+        if (!blocks) {
+            s.step_info.insert(s.step_info.end(), {static_cast<uint32_t>(cur_d), static_cast<uint32_t>(cur_d >> 32), 0u,
+                                                   static_cast<uint32_t>(pend.size())});
+            pend.clear();
+            pend_bytes = 0;
+            return;
+        }
         const size_t off = s.blocks_c128.size();
         uint32_t nterms = 0;
         for (auto &g : pend) {
@@ -232,6 +239,7 @@ Schedule build_schedule(const std::vector<MatrixTerm> &terms, uint32_t nqubits, 
         }
     }
     flush();
+    if (!blocks) return s;
     // complex64 blocks: same layout, weights as two floats + 8 pad bytes
     s.blocks_c64 = s.blocks_c128;
     for (size_t i = 0; i + 4 <= s.step_info.size(); i += 4) {
@@ -356,7 +364,7 @@ void tabulate(std::vector<SignedWeight> rest, std::vector<SignedWeight> &singles
                 for (uint32_t dim = 0; dim < 4; ++dim) {
                     uint32_t best_v = 0;
                     size_t best_new = 0;
-                    const size_t stride = std::max<size_t>(1, rest.size() / 32);
+                    const size_t stride = std::max<size_t>(1, rest.size() / 16);
                     for (size_t i = 0; i < rest.size(); i += stride) {
                         const uint32_t v = rest[i].zs ^ z0;
                         AffineSpan probe = cur;
@@ -560,7 +568,7 @@ RingSchedule build_ring_schedule(const std::vector<MatrixTerm> &terms, uint32_t 
                 ++r.runs;
                 if (++run_index % kRingFoldRuns == 0) {
                     word |= kRingFold;
-                    cur_coset = -1;
+                    if (!c128) cur_coset = -1;
                 }
             }
             if (i < singles.size())

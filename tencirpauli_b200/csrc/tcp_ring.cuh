@@ -247,12 +247,14 @@ __device__ __forceinline__ void ring_walk(const unsigned char *blk, const typena
             ring_dispatch<E, R>(dsum, word, xv, sums.acc);
             dsum = R(0);
             // FP32: fold the running partial sums into the compensated row
-            // sums (every tcp::kRingFoldRuns runs, before a new coset)
+            // sums (every tcp::kRingFoldRuns runs)
             if constexpr (sizeof(R) == 4) {
                 if (word & tcp::kRingFold) {
                     sums.fold();
+                    if constexpr (G::kTmem) {
 #pragma unroll
-                    for (int j = 0; j < E; ++j) xv[j] = C{0.f, 0.f};  // dead: a new coset follows
+                        for (int j = 0; j < E; ++j) xv[j] = C{0.f, 0.f};  // dead: a new coset follows
+                    }
                 }
             }
         }

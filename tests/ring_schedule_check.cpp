@@ -51,7 +51,7 @@ static bool check(const char *name, uint32_t n, const std::vector<tcp::MatrixTer
         const uint32_t low = (1u << shape.low) - 1u;
         return (j & low) | (t << shape.low) | ((j >> shape.low) << (shape.low + shape.log_threads));
     };
-    const tcp::RingSchedule r = tcp::build_ring_schedule(terms, n, shape, !c64 || shape.low == 0);
+    const tcp::RingSchedule r = tcp::build_ring_schedule(terms, n, shape, shape.low == 0);
     if (r.tile_bits != S) return fail_line(name, "no ring schedule");
     const std::vector<uint8_t> &blocks = c64 ? r.blocks_c64 : r.blocks_c128;
     std::mt19937_64 rng(5);
@@ -102,7 +102,7 @@ static bool check(const char *name, uint32_t n, const std::vector<tcp::MatrixTer
                     if (++unfolded > tcp::kRingFoldRuns) return fail_line(name, "too many runs without a fold");
                     if (word & tcp::kRingFold) {
                         unfolded = 0;
-                        src = nullptr;  // a new coset follows
+                        if (shape.low) src = nullptr;  // a new coset follows
                     }
                 }
                 if (sum != 0.0) return fail_line(name, "a block ends inside a run");
@@ -135,7 +135,9 @@ int main() {
         // complex128: T products of FP64 weights; complex64: weights rounded to FP32
         for (const tcp::RingShapeBits shape : tcp::kRingShapes) {
             if (n < shape.tile_bits) continue;
-            if (!check<double>(name, n, t, shape, 1e-13) || !check<float>(name, n, t, shape, 1e-6)) return false;
+            // the 8192-row schedule has complex64 blocks only
+            if (shape.low == 0 && !check<double>(name, n, t, shape, 1e-13)) return false;
+            if (!check<float>(name, n, t, shape, 1e-6)) return false;
         }
         return true;
     };
