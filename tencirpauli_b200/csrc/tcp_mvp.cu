@@ -55,7 +55,7 @@ namespace {
 //    warp's chain of record load, sign, branch and multiply-adds is, with four
 //    warps per scheduler to hide it.  So the work per row counts: D is summed
 //    once per run and thread instead of multiplying every term into every row
-//    (2,000 random words on 28 qubits, complex128: 210 ms before, 169 now;
+//    (2,000 random words on 28 qubits, complex128: 210 ms before, 169 to 175 now;
 //    Jordan-Wigner operator on 20 qubits: 30.7 before, 6.4 ms now), and 16 rows
 //    per thread halve the record walks per row (complex64, 26 qubits: 43.3 ms
 //    before, 38.4 with 8 rows, 24.5 with 16).  16 rows of complex64 with their
