@@ -15,7 +15,6 @@ namespace tcpdev {
 constexpr int kLogThreads = 9;               // 512 threads per CTA
 constexpr int kThreads = 1 << kLogThreads;
 constexpr int kLogRowsC128 = 3;              // 8 rows per thread  -> 4096-row tile
-constexpr int kLogRowsC64 = 3;               // 8 rows per thread  -> 4096-row tile
 constexpr uint32_t kTileBitsC128 = kLogThreads + kLogRowsC128;
 constexpr unsigned long long kWaitLimitNs = 2000000000ull;  // 2 s bound on any device wait
 constexpr uint32_t kCompensateGroups = 4;   // FP32: groups per Kahan fold
@@ -215,15 +214,6 @@ template <> __device__ __forceinline__ float2 record_weight<float>(const unsigne
     return *reinterpret_cast<const float2 *>(rec + 16);
 }
 
-// Flip the sign of w when bit `bit` of `pattern` is set (an integer op on the
-// sign bit; `bit` is a compile-time constant after unrolling).
-__device__ __forceinline__ double flip_if(double w, uint32_t pattern, int bit) {
-    const int hi = __double2hiint(w) ^ static_cast<int>((pattern << (31 - bit)) & 0x80000000u);
-    return __hiloint2double(hi, __double2loint(w));
-}
-__device__ __forceinline__ float flip_if(float w, uint32_t pattern, int bit) {
-    return __int_as_float(__float_as_int(w) ^ static_cast<int>((pattern << (31 - bit)) & 0x80000000u));
-}
 // Flip the sign of w when `odd` (0 or 1) is set.
 __device__ __forceinline__ double flip_by(double w, uint32_t odd) {
     return __hiloint2double(__double2hiint(w) ^ static_cast<int>(odd << 31), __double2loint(w));
