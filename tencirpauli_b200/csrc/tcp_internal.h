@@ -152,6 +152,7 @@ struct RingSchedule {
     uint32_t log_threads = 0;
     uint64_t cosets = 0;               // coset loads per output tile
     uint64_t runs = 0;                 // runs per output tile
+    uint64_t work = 0;                 // steps spent on finding the sign tables
     uint32_t max_block_bytes = 0;      // largest step block
     // 4 words per step: d, complex128 block offset / 16, complex64 block
     // offset / 16, complex128 block bytes / 16 | complex64 block bytes / 16 << 16
