@@ -42,6 +42,7 @@
 
 #include "../../include/tcp_sector.h"
 #include "tcp_internal.h"
+#include "tcp_u1_rank.h"
 
 using tcp::fail;
 
@@ -620,7 +621,7 @@ __global__ void __launch_bounds__(kU1Threads, kU1PairBlocks)
                         j = high + tab[a.l_off + (src & a.lmask)];
                     else if constexpr (RK == 2 && WHERE == 1)
                         j = low + tab[a.h_off + (src >> a.rL)];
-                    else
+                    else  // in the tables for dead pairs too: tcp::u1_table_entries
                         j = static_cast<uint32_t>(rank_any<RK, uint32_t, uint32_t>(src, tab, p, a));
                     xv[u] = C{};
                     if (t != 0u && t != r.x) xv[u] = x[j];
@@ -1325,24 +1326,8 @@ int upload(tcp_u1_plan *p) {
     U1Apply fast{};
     if (p->basis32) {
         const uint32_t n = p->n, k = p->k;
-        uint32_t T_ = 0, M_ = 0, L_ = 0;
-        if (n <= 24) {
-            L_ = n / 2;
-            T_ = n - L_;
-        } else {
-            size_t best = ~size_t(0);
-            for (uint32_t a = 1; a + 2 <= n; ++a)
-                for (uint32_t b = 1; a + b + 1 <= n; ++b) {
-                    const uint32_t c = n - a - b;
-                    const size_t e = (size_t(1) << a) + (std::min(k, a) + 1) * (size_t(1) << b) + (size_t(1) << c);
-                    if (e < best) {
-                        best = e;
-                        T_ = a;
-                        M_ = b;
-                        L_ = c;
-                    }
-                }
-        }
+        const tcp::U1Split split = tcp::u1_split(n, k);
+        const uint32_t T_ = split.top, M_ = split.mid, L_ = split.low;
         const uint32_t lowbits = M_ + L_;  // bits below the top part
         std::vector<uint32_t> H(size_t(1) << T_), Lr(size_t(1) << L_), Mid;
         {
@@ -1356,7 +1341,7 @@ int upload(tcp_u1_plan *p) {
             }
         }
         if (M_) {
-            const uint32_t rows = std::min(k, T_) + 1;
+            const uint32_t rows = tcp::u1_mid_rows(k, T_);
             Mid.assign(size_t(rows) << M_, 0);
             for (uint32_t a = 0; a < rows; ++a) {
                 uint64_t acc = 0;
@@ -1378,6 +1363,7 @@ int upload(tcp_u1_plan *p) {
         ftab.insert(ftab.end(), H.begin(), H.end());
         ftab.insert(ftab.end(), Mid.begin(), Mid.end());
         ftab.insert(ftab.end(), Lr.begin(), Lr.end());
+        ftab.resize(tcp::u1_table_entries(split, k), 0u);
         fast.ftab_bytes = 4 * ftab.size();
     }
     // Pair view: every group a real constant on two qubits, none general.
