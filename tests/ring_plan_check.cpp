@@ -1,11 +1,12 @@
 // Properties of the ring schedules beyond the sums they give: the work of
-// building them.  Built and run by tests/test_ring_plan_cpu.py with the name of
+// building them and the folds of the complex64 sums.  Built and run by tests/test_ring_plan_cpu.py with the name of
 // the check; exits non-zero on the first failure.
 #include <algorithm>
 #include <cmath>
 #include <cstdio>
 #include <cstring>
 #include <random>
+#include <utility>
 #include <vector>
 
 #include "../tencirpauli_b200/csrc/tcp_internal.h"
@@ -108,9 +109,82 @@ static int work() {
     return 0;
 }
 
+// Jordan-Wigner-like, lattice and random operators on n qubits.
+static std::vector<std::pair<const char *, std::vector<MatrixTerm>>> operators(uint32_t n) {
+    std::vector<std::pair<const char *, std::vector<MatrixTerm>>> out;
+    std::vector<MatrixTerm> t;
+    for (uint32_t q = 0; q < n; ++q) {
+        const uint64_t m = 1ull << q | 1ull << (q + 1) % n;
+        t.push_back({m, 0, 0.25, 0.0});
+        t.push_back({m, m, -0.25, 0.0});
+        t.push_back({0, m, 0.25, 0.0});
+        t.push_back({0, 1ull << q, 0.5 * normal(rng), 0.0});
+    }
+    out.emplace_back("lattice", t);
+    t.clear();
+    for (int k = 0; k < 600; ++k) {
+        uint64_t x = 0, z = 0;
+        for (int j = 0; j < 2 + k % 3; ++j) {
+            const uint64_t q = 1ull << rng() % n, letter = rng() % 3;
+            if (letter < 2) x |= q;
+            if (letter > 0) z |= q;
+        }
+        t.push_back({x, z, normal(rng), k % 7 ? 0.0 : normal(rng)});
+    }
+    out.emplace_back("random", t);
+    t.clear();
+    for (int k = 0; k < 150; ++k) {
+        uint64_t m = 0;
+        while (__builtin_popcountll(m) < 4) m |= 1ull << rng() % n;
+        const uint64_t string = rng() & ((1ull << n) - 1) & ~m;
+        for (uint64_t u = m;; u = (u - 1) & m) {
+            if (__builtin_popcountll(u) % 2 == 0) t.push_back({m, string ^ u, normal(rng), 0.0});
+            if (u == 0) break;
+        }
+    }
+    for (uint32_t a = 0; a < n; ++a)
+        for (uint32_t b = 0; b <= a; ++b) t.push_back({0, 1ull << a | 1ull << b, normal(rng), 0.0});
+    out.emplace_back("two-body", t);
+    return out;
+}
+
+// complex64: the kernel carries its partial sums from step to step, so a fold is
+// due every kRingFoldRuns runs of the whole schedule, not of a step.  (The last
+// fold, after the last step, is the kernel's own.)
+static int folds() {
+    for (uint32_t n : {14u, 22u}) {
+        for (const auto &op : operators(n)) {
+            for (const tcp::RingShapeBits shape : tcp::kRingShapes) {
+                const tcp::RingSchedule r = tcp::build_ring_schedule(op.second, n, shape, shape.low == 0);
+                uint32_t unfolded = 0, most = 0;
+                uint64_t runs = 0;
+                for (size_t st = 0; st < r.step_info.size(); st += 4) {
+                    const uint8_t *p = r.blocks_c64.data() + size_t(r.step_info[st + 2]) * 16;
+                    uint32_t left = word32(p);
+                    for (p += 16; left; --left) {
+                        const uint32_t word = word32(p + 4);
+                        p += tcp::ring_record_bytes((word & tcp::kRingKindMask) >> tcp::kRingKindShift, 4);
+                        if (!(word & tcp::kRingLast)) continue;
+                        ++runs;
+                        most = std::max(most, ++unfolded);
+                        if (word & tcp::kRingFold) unfolded = 0;
+                    }
+                }
+                if (most > tcp::kRingFoldRuns || runs != r.runs || runs <= tcp::kRingFoldRuns) {
+                    std::printf("%s, %u qubits: %u of %llu runs without a fold\n", op.first, n, most,
+                                static_cast<unsigned long long>(runs));
+                    return 1;
+                }
+            }
+        }
+    }
+    return 0;
+}
+
 int main(int argc, char **argv) {
     const char *check = argc > 1 ? argv[1] : "";
     if (!std::strcmp(check, "work")) return work();
+    if (!std::strcmp(check, "folds")) return folds();
     std::printf("unknown check\n");
     return 2;
 }

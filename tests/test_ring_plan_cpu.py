@@ -1,5 +1,6 @@
 """Properties of the ring schedules (ring_plan_check.cpp) on the CPU: building
-one takes work linear in the number of terms, whatever the length of a run."""
+one takes work linear in the number of terms, whatever the length of a run, and
+the complex64 sums are folded in time across the steps of a schedule."""
 
 from __future__ import annotations
 
@@ -27,7 +28,7 @@ def checker(tmp_path_factory):
     return exe
 
 
-@pytest.mark.parametrize("check", ["work"])
+@pytest.mark.parametrize("check", ["work", "folds"])
 def test_ring_plans(checker: str, check: str) -> None:
     proc = subprocess.run([checker, check], capture_output=True, text=True, timeout=300)
     assert proc.returncode == 0, proc.stdout[-2000:]
