@@ -561,13 +561,16 @@ __global__ void __launch_bounds__(kU1Threads) k_u1_apply(U1Dev p, U1Apply a, siz
 // (exchange, hopping): the usual lattice and one-body operators.  A pair is
 // live where its two bits differ, and a live group is one multiply-add by
 // +-C.  Against the general kernel this drops, per row and group, the popcount
-// of the live test, the complex product of a real constant and the branch
-// around a dead group (whose value is not loaded, and added as 0 C); and with
+// of the live test and the complex product of a real constant; and with
 // two-level ranks a pair inside the low (high) half of the state changes one
 // table lookup only, so the groups are sorted into classes: low, high, both,
-// each without and with a sign mask z_out.  What remains is issue and the
-// gathers from L2 (4 x 6 J1-J2 half filling, complex128: 376 us before, 268
-// now; 4 groups in flight 273, 8 at 3 blocks per SM 277).
+// each without and with a sign mask z_out.  The value of a dead pair is not
+// loaded; complex128 adds it as 0 C, which is cheaper than a branch around it,
+// complex64 leaves it out of its compensated sum, which would turn an infinite
+// sum into NaN.  What remains is issue and the gathers from L2.  Half filling of
+// the 4 x 6 J1-J2 lattice: complex128 268 us (general kernel 376; 4 groups in
+// flight 273, 8 at 3 blocks per SM 277), complex64 258 (general kernel 369; with
+// complex products of the real constants 275).
 // Three-level ranks (n > 24) use the "both" classes alone.
 constexpr int kU1PairBlocks = 4, kPairUnroll = 6;  // resident blocks per SM; groups in flight
 template <typename R> __device__ __forceinline__ R pair_value(uint4 r);
@@ -575,6 +578,13 @@ template <> __device__ __forceinline__ double pair_value<double>(uint4 r) {
     return __hiloint2double(static_cast<int>(r.w), static_cast<int>(r.z));
 }
 template <> __device__ __forceinline__ float pair_value<float>(uint4 r) { return __uint_as_float(r.z); }
+
+// Compensated FP32 sum += w v.
+__device__ __forceinline__ void kahan_real(float &sum, float &comp, float w, float v) {
+    const float y = fmaf(w, v, -comp), t = sum + y;
+    comp = (t - sum) - y;
+    sum = t;
+}
 
 template <typename R, int RK, bool DIAG>
 __global__ void __launch_bounds__(kU1Threads, kU1PairBlocks)
@@ -612,6 +622,7 @@ __global__ void __launch_bounds__(kU1Threads, kU1PairBlocks)
             for (uint32_t g = g0; g < g1; g += U) {
                 C xv[U];
                 R v[U];
+                bool live[U];
 #pragma unroll
                 for (int u = 0; u < U; ++u) {
                     const uint4 r = rec[g + u];
@@ -624,7 +635,8 @@ __global__ void __launch_bounds__(kU1Threads, kU1PairBlocks)
                     else  // in the tables for dead pairs too: tcp::u1_table_entries
                         j = static_cast<uint32_t>(rank_any<RK, uint32_t, uint32_t>(src, tab, p, a));
                     xv[u] = C{};
-                    if (t != 0u && t != r.x) xv[u] = x[j];
+                    live[u] = t != 0u && t != r.x;
+                    if (live[u]) xv[u] = x[j];
                     v[u] = pair_value<R>(r);
                     if (SIGNED && (__popc(r.y & b) & 1)) v[u] = -v[u];
                 }
@@ -634,7 +646,9 @@ __global__ void __launch_bounds__(kU1Threads, kU1PairBlocks)
                         ar = fma(v[u], xv[u].x, ar);
                         ai = fma(v[u], xv[u].y, ai);
                     } else {
-                        cmac<R, C>(ar, ai, cr, ci, v[u], R(0), xv[u]);
+                        if (!live[u]) continue;
+                        kahan_real(ar, cr, v[u], xv[u].x);
+                        kahan_real(ai, ci, v[u], xv[u].y);
                     }
                 }
             }
