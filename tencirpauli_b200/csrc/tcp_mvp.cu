@@ -338,9 +338,10 @@ template <> struct SmallAcc<float> {  // FP32 products, Kahan-compensated sums
         Acc<float>::kahan(re, cre, __fmaf_rn(w.x, v.x, -__fmul_rn(w.y, v.y)));
         Acc<float>::kahan(im, cim, __fmaf_rn(w.x, v.y, __fmul_rn(w.y, v.x)));
     }
+    // The compensation of an infinite sum is not finite and stays out of it.
     __device__ __forceinline__ double2 sum() const {
-        return make_double2(static_cast<double>(re) - static_cast<double>(cre),
-                            static_cast<double>(im) - static_cast<double>(cim));
+        return make_double2(static_cast<double>(re) - (isfinite(cre) ? static_cast<double>(cre) : 0.0),
+                            static_cast<double>(im) - (isfinite(cim) ? static_cast<double>(cim) : 0.0));
     }
 };
 
