@@ -291,7 +291,7 @@ template <> struct Acc<float> {
 // the scalar instruction), so one instruction serves both components.  Two
 // running partial sums -- p for real weights (w x) and q for imaginary
 // weights (w x, whose contribution is i q) -- take the same instruction form;
-// fold() adds p + i q to the Kahan-compensated row sum, which the kernel keeps
+// fold() adds p + i q to the compensated row sum, which the kernel keeps
 // in registers (8 rows per thread) or in tensor memory (16 rows).
 template <typename R> struct RingAcc;
 template <> struct RingAcc<double> : Acc<double> {};
@@ -326,15 +326,20 @@ template <> struct RingAcc<float> {
     uint64_t p = 0, q = 0;  // running partial sums of real / imaginary weights
     __device__ __forceinline__ void add_real(float w, float2 v) { p = fma2(pack2(w, w), pack2(v.x, v.y), p); }
     __device__ __forceinline__ void add_imag(float w, float2 v) { q = fma2(pack2(w, w), pack2(v.x, v.y), q); }
-    // Fold p + i q into the Kahan sum s with compensation c, both (re, im).
+    // Add p + i q to the row sum s and the rounding error of that to c, both (re,
+    // im).  c is not fed back into the sum (it would turn an infinite sum into NaN
+    // at the next fold) but added once, by value().
     __device__ __forceinline__ void fold(uint64_t &s, uint64_t &c) {
         const float2 qq = unpack2(q);
         const uint64_t term = add2(p, pack2(-qq.y, qq.x));  // p + i q
-        const uint64_t yv = sub2(term, c);
-        const uint64_t tv = add2(s, yv);
-        c = sub2(sub2(tv, s), yv);
-        s = tv;
+        const uint64_t sum = add2(s, term);
+        c = add2(c, add2(sub2(s, sum), term));
+        s = sum;
         p = q = 0;
+    }
+    __device__ __forceinline__ static float2 value(uint64_t s, uint64_t c) {
+        const float2 sv = unpack2(s), cv = unpack2(c);
+        return make_float2(sv.x + (isfinite(cv.x) ? cv.x : 0.f), sv.y + (isfinite(cv.y) ? cv.y : 0.f));
     }
 };
 

@@ -140,7 +140,7 @@ constexpr uint32_t kRingFlipShift = 10;       // 4 bits: negate the loaded value
 constexpr uint32_t kRingFlipMask = 15u << kRingFlipShift;
 constexpr uint32_t kRingMaskShift = 14;       // 9 bits: m_lo
 
-constexpr uint32_t kRingFoldRuns = 16;        // complex64: runs per Kahan fold
+constexpr uint32_t kRingFoldRuns = 16;        // complex64: runs per fold
 
 // Bytes of a record of each kind.
 constexpr uint32_t ring_record_bytes(uint32_t kind, uint32_t weight_bytes) {

@@ -59,8 +59,8 @@ namespace {
 //    Jordan-Wigner operator on 20 qubits: 30.7 before, 6.4 ms now), and 16 rows
 //    per thread halve the record walks per row (complex64, 26 qubits: 43.3 ms
 //    before, 38.4 with 8 rows, 24.5 with 16).  16 rows of complex64 with their
-//    Kahan sums would need 128 registers beside the 32 of the loaded values;
-//    the Kahan sums, touched every kRingFoldRuns runs only, live in tensor
+//    compensated sums would need 128 registers beside the 32 of the loaded values;
+//    the compensated sums, touched every kRingFoldRuns runs only, live in tensor
 //    memory (64 columns per warp), which this kernel otherwise has no use for.
 //    256 threads of 16 rows in 4096-row tiles measured slower than 512 of 8
 //    (complex128 22.9 against 21.2 ms, complex64 19.7 against 18.1 ms, 25 qubits).

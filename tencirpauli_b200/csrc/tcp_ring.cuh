@@ -127,7 +127,7 @@ __device__ __forceinline__ void ring_dispatch(R d, uint32_t word, const typename
 #undef TCP_RING_CASE
 }
 
-// The thread's accumulators and, complex64, its Kahan sums.
+// The thread's accumulators and, complex64, its compensated sums.
 template <typename R, int SHAPE> struct RingSums {
     static constexpr int E = RingGeo<R, SHAPE>::kRows;
     RingAcc<R> acc[E];
@@ -143,7 +143,7 @@ template <> struct RingSums<float, 0> {
 #pragma unroll
         for (int j = 0; j < E; ++j) acc[j].fold(s[j], c[j]);
     }
-    __device__ __forceinline__ float2 value(int j) const { return unpack2(s[j]); }
+    __device__ __forceinline__ float2 value(int j) const { return RingAcc<float>::value(s[j], c[j]); }
 };
 // 16 rows: (s, c) of rows 4 k .. 4 k + 3 in 16 tensor-memory columns of the
 // thread's lane.
@@ -176,7 +176,7 @@ template <> struct RingSums<float, 1> {
         uint64_t v[8];
         tmem_load8(tmem + 16u * k, v);
 #pragma unroll
-        for (uint32_t j = 0; j < 4; ++j) out[j] = unpack2(v[2 * j]);
+        for (uint32_t j = 0; j < 4; ++j) out[j] = RingAcc<float>::value(v[2 * j], v[2 * j + 1]);
     }
 };
 
