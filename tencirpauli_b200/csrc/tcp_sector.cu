@@ -1082,6 +1082,16 @@ std::string bytes_str(unsigned __int128 v) {
     return v >> 64 ? std::string("more than 2^64") : std::to_string(static_cast<uint64_t>(v));
 }
 
+// Shared-memory opt-in of a staged kernel and its resident blocks per SM with
+// `smem` bytes.  The opt-in belongs to the kernel, not to the launch: it is the
+// same for every plan, so that a thread never lowers it under another's launch.
+template <typename K> int opt_in_smem(K *kernel, size_t smem, int &per_sm) {
+    cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(kU1SmemMax));
+    if (e != cudaSuccess) return cuda_fail(e, "cudaFuncSetAttribute");
+    e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, kU1Threads, smem);
+    return e == cudaSuccess ? TCP_OK : cuda_fail(e, "cudaOccupancyMaxActiveBlocksPerMultiprocessor");
+}
+
 template <typename R, typename ST, typename IT, int RK, bool SM, bool DIAG>
 int launch_apply_v(const tcp_u1_plan *p, const void *x, void *y, cudaStream_t s, uint64_t row0, uint64_t row1) {
     using C = typename Cplx<R>::T;
@@ -1092,11 +1102,9 @@ int launch_apply_v(const tcp_u1_plan *p, const void *x, void *y, cudaStream_t s,
     if (SM) {
         // one wave of resident CTAs: each CTA stages the tables once
         smem = sizeof(R) == 8 ? p->smem_c128 : p->smem_c64;
-        cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));
-        if (e != cudaSuccess) return cuda_fail(e, "cudaFuncSetAttribute");
         int per_sm = 0;
-        e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, kU1Threads, smem);
-        if (e != cudaSuccess) return cuda_fail(e, "cudaOccupancyMaxActiveBlocksPerMultiprocessor");
+        const int st = opt_in_smem(kern, smem, per_sm);
+        if (st) return st;
         grid = std::min<int>(grid, std::max(per_sm, 1) * std::max(g_sms, 1));
     }
     kern<<<grid, kU1Threads, smem, s>>>(p->dev, p->app, tab_bytes, static_cast<const C *>(x), static_cast<C *>(y), row0,
@@ -1110,15 +1118,13 @@ int launch_pairs_v(const tcp_u1_plan *p, const void *x, void *y, cudaStream_t s,
     using C = typename Cplx<R>::T;
     auto kern = k_u1_pairs<R, RK, DIAG>;
     const size_t smem = 16ull * p->app.pair_seg[6] + p->app.ftab_bytes;
-    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));
-    if (e != cudaSuccess) return cuda_fail(e, "cudaFuncSetAttribute");
     int per_sm = 0;
-    e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, kU1Threads, smem);
-    if (e != cudaSuccess) return cuda_fail(e, "cudaOccupancyMaxActiveBlocksPerMultiprocessor");
+    const int st = opt_in_smem(kern, smem, per_sm);
+    if (st) return st;
     // one wave of resident CTAs: each CTA stages the tables once
     const int grid = std::min<int>(grid_for(row1 - row0), std::max(per_sm, 1) * std::max(g_sms, 1));
     kern<<<grid, kU1Threads, smem, s>>>(p->dev, p->app, static_cast<const C *>(x), static_cast<C *>(y), row0, row1);
-    e = cudaGetLastError();
+    const cudaError_t e = cudaGetLastError();
     return e == cudaSuccess ? TCP_OK : cuda_fail(e, "sector MVP kernel launch");
 }
 
