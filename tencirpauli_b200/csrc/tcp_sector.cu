@@ -1439,10 +1439,16 @@ int upload(tcp_u1_plan *p) {
         {pairs.data(), 4ull * pairs.size(), 0},
         {pairsf.data(), 4ull * pairsf.size(), 0},
     };
-    size_t off = 0;
-    for (auto &pc : pieces) {
-        pc.off = off;
-        off += (pc.bytes + 255) / 256 * 256;
+    // The host's pieces first, so that one copy brings them all: each blocking copy
+    // of a small piece takes 7 us, whatever its size.
+    size_t off = 0, copied = 0;
+    for (const bool from_host : {true, false}) {
+        for (auto &pc : pieces) {
+            if ((pc.src != nullptr) != from_host) continue;
+            pc.off = off;
+            off += (pc.bytes + 255) / 256 * 256;
+        }
+        if (from_host) copied = off;
     }
     void *block = nullptr;
     cudaError_t e = tcp::injected_alloc_failure() ? cudaErrorMemoryAllocation : cudaMalloc(&block, std::max<size_t>(off, 256));
@@ -1451,14 +1457,13 @@ int upload(tcp_u1_plan *p) {
         return fail(TCP_ERR_ALLOCATION, "device allocation of the sector plan (" + std::to_string(off) + " bytes) failed");
     }
     unsigned char *base = static_cast<unsigned char *>(block);
-    for (auto &pc : pieces) {
-        if (pc.src && pc.bytes) {
-            e = cudaMemcpy(base + pc.off, pc.src, pc.bytes, cudaMemcpyHostToDevice);
-            if (e != cudaSuccess) {
-                cudaFree(block);
-                return cuda_fail(e, "uploading the sector plan");
-            }
-        }
+    std::vector<unsigned char> staging(copied, 0);
+    for (const auto &pc : pieces)
+        if (pc.src && pc.bytes) std::memcpy(staging.data() + pc.off, pc.src, pc.bytes);
+    e = cudaMemcpy(base, staging.data(), copied, cudaMemcpyHostToDevice);
+    if (e != cudaSuccess) {
+        cudaFree(block);
+        return cuda_fail(e, "uploading the sector plan");
     }
     p->block = block;
     p->block_bytes = off;
