@@ -232,7 +232,7 @@ Schedule build_schedule(const std::vector<MatrixTerm> &terms, uint32_t nqubits, 
                 pend.push_back(Pending{m_in, g, {}});
                 pend_bytes += kGroupRecBytes;
             }
-            pend.back().terms.push_back(order[t]);
+            if (blocks) pend.back().terms.push_back(order[t]);
             pend_bytes += kTermRecBytes;
         }
     }
