@@ -102,6 +102,27 @@ def _issue_roofline(kernel: str, workload: str, kernel_ms: float, clocks: Dict[s
             "instructions_per_launch": inst, "source": "profiles/instructions.txt (ncu smsp__inst_executed.sum)"}
 
 
+def _smem_roofline(dtype: str, n: int, cosets: int, ring_steps: int, kernel_ms: float, smem_rate: float) -> Dict[str, Any]:
+    """Shared-memory operand rate of k_ring against the probed one.  The plan
+    counts cosets and steps of the 4096-row tiles, which complex128 runs;
+    complex64 runs 8192-row tiles, whose operands the plan does not count, so
+    only the peak is given."""
+    out: Dict[str, Any] = {
+        "achieved": None,
+        "peak": smem_rate / 1e12,
+        "unit": "TB/s",
+        "frac": None,
+        "peak_source": "tcp_probe_smem_rate: 16-byte shared-memory reads in the kernel's pattern on every SM "
+        "of this GPU, best of 5",
+    }
+    if dtype == "c128":
+        nbytes = (1 << n) * (cosets + ring_steps) * 16
+        rate = nbytes / (kernel_ms / 1000.0)
+        out.update(achieved=rate / 1e12, frac=rate / smem_rate, bytes_per_launch=nbytes,
+                   units=f"2^{n} rows x ({cosets} coset operands + {ring_steps} tile fills) x 16 B")
+    return out
+
+
 def manifest(with_gpu: bool = True) -> Dict[str, Any]:
     """What produced a bench line: the library's build record (source commit,
     nvcc release), a digest of the sources as they ran, host core count,
@@ -717,20 +738,20 @@ def run_sector(args: argparse.Namespace) -> None:
     peaks = _measured_peaks()
     b_alg = dim * (4 + 16 + 2 * elem)  # basis word, diagonal, x, y
     achieved = b_alg / (ms / 1e3) / 1e9
-    # k_u1_apply is bound by instruction issue (gathers and table lookups
+    # k_u1_pairs is bound by instruction issue (gathers and table lookups
     # in flight, not bytes): its roofline is the issue rate, with the
     # compulsory HBM bytes beside it
     hbm = {"achieved": achieved, "peak": peaks["hbm_gbs"], "unit": "GB/s", "frac": achieved / peaks["hbm_gbs"],
            "bytes_per_launch": b_alg, "peak_source": peaks["source"]}
-    issue = _issue_roofline("k_u1_apply", f"j1j2_{lx}x{ly}_half_{args.dtype}", ms, clocks)
+    issue = _issue_roofline("k_u1_pairs", f"j1j2_{lx}x{ly}_half_{args.dtype}", ms, clocks)
     if issue is not None:
         sector_roofline = dict(bound="issue", **{k: issue[k] for k in ("achieved", "peak", "unit", "frac")},
-                               kernel="k_u1_apply", kernel_ms=ms, instructions_per_launch=issue["instructions_per_launch"],
+                               kernel="k_u1_pairs", kernel_ms=ms, instructions_per_launch=issue["instructions_per_launch"],
                                peak_source="4 warp instructions per SM clock x SMs x sampled SM clock; "
                                + issue["source"], hbm=hbm)
     else:
         sector_roofline = dict(bound="issue (instruction count not profiled for this lattice; HBM shown)",
-                               **{k: hbm[k] for k in ("achieved", "peak", "unit", "frac")}, kernel="k_u1_apply",
+                               **{k: hbm[k] for k in ("achieved", "peak", "unit", "frac")}, kernel="k_u1_pairs",
                                kernel_ms=ms, bytes_per_launch=b_alg, peak_source=peaks["source"])
     line = {
         "metric": "Sector MVP amplitude-terms/s",
@@ -1127,24 +1148,12 @@ def main() -> None:
         info = native.info
         f_alg = dim * (2 * T + 8 * G)
         f_ach = f_alg / (kern_ms / 1000.0)
-        smem_bytes = dim * (int(info.cosets) + int(info.ring_steps)) * elem
-        smem_ach = smem_bytes / (kern_ms / 1000.0)
         # The binding resource is instruction issue (the per-record integer
         # chain ahead of the multiply-adds; ncu: issue active about half the
         # cycles, neither the shared-memory nor the FMA pipe saturated), so
         # the main roofline is the issue rate; shared memory, the FMA pipe
         # and HBM are reported beside it.
-        smem_obj = {
-            "achieved": smem_ach / 1e12,
-            "peak": smem_rate / 1e12,
-            "unit": "TB/s",
-            "frac": smem_ach / smem_rate,
-            "peak_source": "tcp_probe_smem_rate: 16-byte shared-memory reads in the kernel's pattern on every SM "
-            "of this GPU, best of 5",
-            "bytes_per_launch": smem_bytes,
-            "units": f"2^{n} rows x ({int(info.cosets)} coset operands + {int(info.ring_steps)} tile fills) x {elem} B"
-            + ("" if args.dtype == "c128" else " (4096-row schedule; the 8192-row tiles that run move fewer)"),
-        }
+        smem_obj = _smem_roofline(args.dtype, n, int(info.cosets), int(info.ring_steps), kern_ms, smem_rate)
         fp_obj = {
             "achieved": f_ach / 1e12,
             "peak": fma_rate / 1e12,
@@ -1169,11 +1178,11 @@ def main() -> None:
                              "instructions_per_launch": issue_obj["instructions_per_launch"],
                              "peak_source": "4 warp instructions per SM clock x SMs x sampled SM clock; " + issue_obj["source"],
                              "smem": smem_obj, "fp": fp_obj, "hbm": hbm_obj}
-        else:  # no committed instruction count for this workload: shared memory leads
-            ring_roofline = {"bound": "smem", **{k: smem_obj[k] for k in ("achieved", "peak", "unit", "frac")},
+        else:  # no committed instruction count for this workload: shared memory leads, or the FMA pipe
+            bound, lead = ("smem", smem_obj) if smem_obj["frac"] is not None else ("fp", fp_obj)
+            ring_roofline = {"bound": bound, **{k: lead[k] for k in ("achieved", "peak", "unit", "frac")},
                              "traffic": traffic, "kernel": kernel_name, "kernel_ms": kern_ms,
-                             "peak_source": smem_obj["peak_source"], "smem_bytes_per_launch": smem_bytes,
-                             "fp": fp_obj, "hbm": hbm_obj}
+                             "peak_source": lead["peak_source"], "smem": smem_obj, "fp": fp_obj, "hbm": hbm_obj}
         line = {
             "metric": METRIC,
             "value": value,
