@@ -128,8 +128,9 @@ struct Schedule {
 // where it ends, where a coset begins (the 8 source values are loaded then)
 // and, complex64, where the partial sums are folded into the compensated row
 // sums (in a schedule without complex128 blocks a new coset follows a fold, so
-// that the 16-row kernel holds no loaded values across it).  Records are 16-byte aligned and the next one is loaded while the
-// present one is applied, so a block leaves 16 bytes of its stage unused.
+// that the 16-row kernel holds no loaded values across it).  Records are 16-byte
+// aligned and the next one is loaded while the present one is applied, so a
+// block leaves 16 bytes of its stage unused.
 constexpr uint32_t kRingImag = 1u << 4;       // bits 0..3: the register permutation a
 constexpr uint32_t kRingKindShift = 5;        // 0 single, 1 / 2 / 3: table of 4 / 8 / 16
 constexpr uint32_t kRingKindMask = 3u << kRingKindShift;
@@ -153,7 +154,6 @@ struct RingSchedule {
     uint64_t cosets = 0;               // coset loads per output tile
     uint64_t runs = 0;                 // runs per output tile
     uint64_t work = 0;                 // steps spent on finding the sign tables
-    uint32_t max_block_bytes = 0;      // largest step block
     // 4 words per step: d, complex128 block offset / 16, complex64 block
     // offset / 16, complex128 block bytes / 16 | complex64 block bytes / 16 << 16
     std::vector<uint32_t> step_info;

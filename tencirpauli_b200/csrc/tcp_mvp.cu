@@ -55,14 +55,14 @@ namespace {
 //    warp's chain of record load, sign, branch and multiply-adds is, with four
 //    warps per scheduler to hide it.  So the work per row counts: D is summed
 //    once per run and thread instead of multiplying every term into every row
-//    (2,000 random words on 28 qubits, complex128: 210 ms before, 169 to 175 now;
-//    Jordan-Wigner operator on 20 qubits: 30.7 before, 6.4 ms now), and 16 rows
-//    per thread halve the record walks per row (complex64, 26 qubits: 43.3 ms
-//    before, 38.4 with 8 rows, 24.5 with 16).  16 rows of complex64 with their
-//    compensated sums would need 128 registers beside the 32 of the loaded values;
-//    the compensated sums, touched every kRingFoldRuns runs only, live in tensor
-//    memory (64 columns per warp), which this kernel otherwise has no use for.
-//    256 threads of 16 rows in 4096-row tiles measured slower than 512 of 8
+//    (2,000 random words on 28 qubits, complex128: 174 ms against 212;
+//    Jordan-Wigner operator on 20 qubits: 6.5 against 30.7), and 16 rows per
+//    thread halve the record walks per row (complex64, 26 qubits: 23.9 ms; 8 rows
+//    took 38.4, and 43.3 with every term multiplied).  16 rows of complex64 with
+//    their compensated sums would need 128 registers beside the 32 of the loaded
+//    values; the compensated sums, touched every kRingFoldRuns runs only, live in
+//    tensor memory (64 columns per warp), which this kernel otherwise has no use
+//    for.  256 threads of 16 rows in 4096-row tiles measured slower than 512 of 8
 //    (complex128 22.9 against 21.2 ms, complex64 19.7 against 18.1 ms, 25 qubits).
 //  * Refills: a producer warp (complex128) or the row warp that releases a
 //    stage last (complex64) has the TMA bulk-copy engine refill it with a later
@@ -501,7 +501,7 @@ constexpr uint64_t kHostChunkRows = uint64_t(1) << 25;  // rows from which the h
 
 size_t align_up(size_t v, size_t a) { return (v + a - 1) / a * a; }
 
-// Step ranges of the source-chunk passes (see DevSchedule::pass_begin): the
+// Step ranges of the source-chunk passes (see RingView::pass_begin): the
 // top kPassBits bits v of each step's outer pattern d, which is
 // non-decreasing in step order because steps are sorted by d.
 void set_passes(const std::vector<uint64_t> &pattern, uint32_t tile_bits, uint32_t nqubits, uint32_t *pass_begin,
@@ -522,7 +522,7 @@ void set_passes(const std::vector<uint64_t> &pattern, uint32_t tile_bits, uint32
     *pass_shift = shift;
 }
 
-// Lay both schedules out in one device allocation.
+// Lay the group view and the ring schedules out in one device allocation.
 int upload(tcp_mvp_plan *p) {
     tcp::Range range("plan upload");
     struct Piece {
@@ -849,7 +849,7 @@ bool page_locked(const void *p) {
 }
 
 // Copies of one host apply.  Page-locked buffers go straight to the DMA
-// engine.  Ordinary buffers of at least two slots go through the staging
+// engine.  Ordinary buffers of at least kStageMinBytes go through the staging
 // ring: the host threads fill a free slot while the DMA engine drains the
 // previous ones (input), or empty a slot whose DMA has landed while later
 // slots are in flight (output), so both directions stay asynchronous to the

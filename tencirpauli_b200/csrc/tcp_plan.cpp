@@ -626,7 +626,6 @@ RingSchedule build_ring_schedule(const std::vector<MatrixTerm> &terms, uint32_t 
             dst.insert(dst.end(), src.begin(), src.end());
             bytes[f] = dst.size() - off[f];
         }
-        r.max_block_bytes = std::max<uint32_t>(r.max_block_bytes, static_cast<uint32_t>(bytes[c128 ? 0 : 1]));
         r.step_info.push_back(cur_d);
         r.step_info.push_back(static_cast<uint32_t>(off[0] / 16));
         r.step_info.push_back(static_cast<uint32_t>(off[1] / 16));

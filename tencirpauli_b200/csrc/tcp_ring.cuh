@@ -9,8 +9,9 @@ namespace tcpdev {
 
 // Geometry of one ring kernel: SHAPE indexes tcp::kRingShapes.
 // Who refills the ring.  complex128: a dedicated producer warp waits on the
-// stages' "empty" barriers and issues the fills (184.6 ms against 191.6 without
-// it for 2,000 random words on 28 qubits).  complex64: no extra warp -- the row
+// stages' "empty" barriers and issues the fills (2,000 random words on 28 qubits:
+// 168 ms against 191 without it; 20-qubit chain: 31 us against 37, in launches one
+// after another).  complex64: no extra warp -- the row
 // warp that releases a stage last issues its refill -- so the 512 threads keep
 // 128 registers for the paired FP32 accumulators.
 template <typename R, int SHAPE> struct RingGeo {
@@ -109,8 +110,9 @@ __device__ __forceinline__ void ring_apply(R d, uint32_t word, const typename Cx
 template <int E, typename R>
 __device__ __forceinline__ void ring_dispatch(R d, uint32_t word, const typename Cx<R>::T (&xv)[E], RingAcc<R> (&acc)[E]) {
     // Most runs have a = 0 (a group rarely flips one of the few register bits):
-    // one test ahead of the switch (complex128, 28 qubits: 175 -> 169 ms).  For
-    // complex64 the test takes real weights along (J1-J2 block: 3.70 -> 3.57 ms).
+    // one test ahead of the switch, which for complex64 takes real weights along
+    // (26 qubits 23.7 ms, 24.0 without it; J1-J2 block 3.57 and 3.71 ms).  complex128
+    // takes the same time with and without it (28 qubits: 168 ms).
     constexpr uint32_t kCommon = static_cast<uint32_t>(E - 1) | (sizeof(R) == 4 ? tcp::kRingImag : 0u);
     if ((word & kCommon) == 0u) {
         ring_apply<0, E, R>(d, sizeof(R) == 4 ? 0u : word, xv, acc);
@@ -184,8 +186,9 @@ template <> struct RingSums<float, 1> {
 // memory, so the compiler must guard each branch on them with convergence
 // barriers (8 of 74 instructions per run).  A warp reduction of the next word,
 // taken while the present run is applied, makes them uniform.  It pays for
-// complex128 (28 qubits: 188 -> 175 ms) and not for complex64, whose runs are
-// shorter (26 qubits: 24.5 -> 26.4 ms).
+// complex128 (28 qubits: 168 ms against 180; Jordan-Wigner operator on 20 qubits:
+// 6.45 against 7.10) and not for complex64, whose runs are shorter (26 qubits: 26.0
+// against 23.7 ms).
 template <typename R> __device__ __forceinline__ uint32_t ring_uniform(uint32_t word) {
     if constexpr (sizeof(R) == 8)
         return __reduce_or_sync(0xffffffffu, word);

@@ -345,8 +345,8 @@ __global__ void __launch_bounds__(kGramThreads, 1)
 
 // Deterministic reduction of the per-block partials: a block takes 32 pairs;
 // warp w adds the partials w, w + 32, ... of each (coalesced across the lanes),
-// then warp 0 adds the 32 sums in warp order.  (One thread per pair walking all
-// 148 partials, as before, took 20 us, most of it load latency; this takes 4.)
+// then warp 0 adds the 32 sums in warp order: 4 us.  (One thread per pair walking
+// all 148 partials takes 20, most of it load latency.)
 constexpr int kGramReduceWarps = 32;
 __global__ void __launch_bounds__(kGramReduceWarps * 32)
     k_gram_reduce(const double2 *__restrict__ partial, uint32_t blocks, uint32_t pairs, double2 *__restrict__ out) {
@@ -637,8 +637,8 @@ __device__ __forceinline__ float act_tanh(float a) {
 // The parameters in the order mlp_eval reads them: per unit o of layer 1 its 8
 // weights, its bias, three zeros, then its column of W2; then b2, w3, b3.
 // Two rows per thread at 64 registers, four blocks of 256 per SM: 506 us for 4
-// residuals of 2^22 complex128 states (one row per thread, before: 690; two rows
-// at 80 registers: 527; three at 80: 762; four at 128 registers: 614; two packed
+// residuals of 2^22 complex128 states (one row per thread: 690; two rows at
+// 80 registers: 527; three at 80: 762; four at 128 registers: 614; two packed
 // in f32x2 with doubled weights: 546).
 constexpr int kEvalThreads = 256, kEvalBlocks = 4, kEvalRows = 2;
 constexpr int kEvalUnit = IN + 4 + HID;
@@ -801,8 +801,8 @@ __global__ void __launch_bounds__(kEvalThreads, kEvalBlocks)
 // takes the units 4 w .. 4 w + 3 of every layer and lane l the samples 4 l ..
 // 4 l + 3: a 16-byte load brings one feature of four samples, and the 109
 // weight-gradient sums of the warp's units stay in each lane's registers
-// across the chunks (12 multiply-adds per load; one thread per parameter, as
-// before, paid two loads for each: 590 us for 1.6 M samples).  The lanes are
+// across the chunks (12 multiply-adds per load: 177 us for 1.6 M samples; one
+// thread per parameter pays two loads for each: 590 us).  The lanes are
 // added by a fixed butterfly at the end, so the result is deterministic; each
 // block writes its gradient partial sum.
 constexpr int kTrainChunk = 128;
