@@ -733,21 +733,21 @@ __device__ __forceinline__ void load_row8(const float *__restrict__ row, bool wi
 
 // Learned correction for k residual vectors: t_j = -exp(c) r_j / den with
 // den = H_ii - theta_j (FP64 diagonal, clamped by eps, exactly as k_jacobi).
-// kEvalRows residuals of a state share its features and every weight load
-// (those past k repeat the last one and are not stored).  The state's features
-// and diagonal are read again per group of residuals rather than held in
-// registers beside the layer-2 sums.
+// kEvalRows residuals of a state share its features and every weight load; what is
+// left of k goes one by one (2^22 states, one residual: 208 us, 251 as half of a
+// pair).  The state's features and diagonal are read again per group of residuals
+// rather than held in registers beside the layer-2 sums.
 __global__ void __launch_bounds__(kEvalThreads, kEvalBlocks)
     k_mlp_precond(const void *__restrict__ R, int r64, uint64_t n, uint32_t k, const float *feat, int wide,
                   const double2 *diag, const double *theta, double scale, double eps, float clamp,
                   const float *__restrict__ wglob, void *__restrict__ T, int t64) {
-    constexpr int V = kEvalRows;
     __shared__ __align__(16) float sw[kEvalWords];
     mlp_stage(sw, wglob);
     __syncthreads();
     for (uint64_t r = blockIdx.x * static_cast<uint64_t>(blockDim.x) + threadIdx.x; r < n;
          r += static_cast<uint64_t>(gridDim.x) * blockDim.x) {
-        for (uint32_t j0 = 0; j0 < k; j0 += V) {
+        auto correct = [&](auto rows, uint32_t j0) {  // residuals j0 .. j0 + V - 1
+            constexpr int V = decltype(rows)::value;
             float own[4][V], shared[4], c[V];  // inputs 0, 1, 2, 7 and 3 .. 6
             {
                 const float *row = feat + r * TCP_FEATURES;
@@ -759,7 +759,7 @@ __global__ void __launch_bounds__(kEvalThreads, kEvalBlocks)
                 for (int v = 0; v < V; ++v) {
                     float x[IN];
                     double den;
-                    state.inputs(theta[min(j0 + v, k - 1u)], eps, x, den);
+                    state.inputs(theta[j0 + v], eps, x, den);
 #pragma unroll
                     for (int i = 0; i < 3; ++i) own[i][v] = x[i];
                     own[3][v] = x[7];
@@ -776,7 +776,6 @@ __global__ void __launch_bounds__(kEvalThreads, kEvalBlocks)
 #pragma unroll
             for (int v = 0; v < V; ++v) {
                 const uint32_t j = j0 + v;
-                if (j >= k) break;
                 const float cj = fminf(fmaxf(c[v], -clamp), clamp);
                 double den = d - theta[j];
                 if (fabs(den) < eps) den = den < 0.0 ? -eps : eps;
@@ -788,7 +787,10 @@ __global__ void __launch_bounds__(kEvalThreads, kEvalBlocks)
                     store_c(T, t64, j * n + r, make_double2(g * rv.x, g * rv.y));
                 }
             }
-        }
+        };
+        uint32_t j0 = 0;
+        for (; j0 + kEvalRows <= k; j0 += kEvalRows) correct(std::integral_constant<int, kEvalRows>{}, j0);
+        for (; j0 < k; ++j0) correct(std::integral_constant<int, 1>{}, j0);
     }
 }
 
