@@ -1046,23 +1046,21 @@ __device__ __forceinline__ double align_g(float c, float den, float clamp) {
     return -exp(cc) / static_cast<double>(den);
 }
 
-// One cluster of kAlignCluster blocks per set: the blocks take the set's states
-// in turn, and the first adds their five sums through distributed shared memory
-// in rank order (a fixed-order tree inside each block), so the sums do not
-// depend on scheduling.  (One block per set left most SMs idle: 280 us for 24
-// sets of 65,536 states.)
-constexpr int kAlignCluster = 8;
-__global__ void __launch_bounds__(kAlignThreads) __cluster_dims__(kAlignCluster, 1, 1)
-    k_align_sums(const float *__restrict__ c, const float *__restrict__ den, const double2 *__restrict__ alpha,
-                 const double *__restrict__ a, const double2 *__restrict__ gamma, const double *__restrict__ E,
-                 const uint64_t *__restrict__ seg_begin, float clamp, double *__restrict__ sums) {
+// The sums of set s: N blocks of THREADS threads take its states in turn, and the
+// first adds their five sums through distributed shared memory in rank order (a
+// fixed-order tree inside each block), so the sums do not depend on scheduling.
+template <int N, int THREADS>
+__device__ __forceinline__ void align_sums(uint32_t s, uint32_t rank, const float *__restrict__ c,
+                                           const float *__restrict__ den, const double2 *__restrict__ alpha,
+                                           const double *__restrict__ a, const double2 *__restrict__ gamma,
+                                           const double *__restrict__ E, const uint64_t *__restrict__ seg_begin,
+                                           float clamp, double *__restrict__ sums) {
     namespace cg = cooperative_groups;
-    __shared__ double red[5][kAlignThreads / 32];
+    __shared__ double red[5][THREADS / 32];
     __shared__ double mine[5];
-    const cg::cluster_group cluster = cg::this_cluster();
-    const uint32_t s = blockIdx.x / kAlignCluster, rank = blockIdx.x % kAlignCluster, t = threadIdx.x;
+    const uint32_t t = threadIdx.x;
     double v[5] = {0.0, 0.0, 0.0, 0.0, 0.0};
-    for (uint64_t i = seg_begin[s] + rank * kAlignThreads + t; i < seg_begin[s + 1]; i += kAlignCluster * kAlignThreads) {
+    for (uint64_t i = seg_begin[s] + rank * THREADS + t; i < seg_begin[s + 1]; i += N * THREADS) {
         const double g = align_g(c[i], den[i], clamp);
         const double2 al = alpha[i], ga = gamma[i];
         v[0] += g * al.x;
@@ -1080,24 +1078,50 @@ __global__ void __launch_bounds__(kAlignThreads) __cluster_dims__(kAlignCluster,
     __syncthreads();
     if (t < 5) {
         double sum = 0.0;
-        for (int q = 0; q < kAlignThreads / 32; ++q) sum += red[t][q];
+        for (int q = 0; q < THREADS / 32; ++q) sum += red[t][q];
         mine[t] = sum;
     }
-    cluster.sync();
-    if (rank == 0 && t < 5) {
+    if constexpr (N > 1) {
+        const cg::cluster_group cluster = cg::this_cluster();
+        cluster.sync();
         double sum = 0.0;
-        for (int q = 0; q < kAlignCluster; ++q) sum += cluster.map_shared_rank(mine, q)[t];
-        red[t][0] = sum;
+        if (rank == 0 && t < 5) {
+            for (int q = 0; q < N; ++q) sum += cluster.map_shared_rank(mine, q)[t];
+        }
+        cluster.sync();  // no block leaves, or overwrites its sums, while they are being read
+        if (rank == 0 && t < 5) mine[t] = sum;
     }
-    cluster.sync();  // no block leaves while its sums are being read
+    __syncthreads();
     if (rank == 0 && t == 0) {
         double *q = sums + static_cast<size_t>(s) * kAlignWords;
 #pragma unroll
-        for (int k = 0; k < 5; ++k) q[k] = red[k][0];
-        const double D = fmax(red[2][0] - (red[3][0] * red[3][0] + red[4][0] * red[4][0]), 1e-300);
-        const double A2 = red[0][0] * red[0][0] + red[1][0] * red[1][0];
+        for (int k = 0; k < 5; ++k) q[k] = mine[k];
+        const double D = fmax(mine[2] - (mine[3] * mine[3] + mine[4] * mine[4]), 1e-300);
+        const double A2 = mine[0] * mine[0] + mine[1] * mine[1];
         q[5] = 1.0 - A2 / (E[s] * D);
     }
+}
+
+// One block per set, or a cluster of eight.  A cluster takes 0.08 us to launch and
+// meet, whatever its set; a block walks its set at 3.8 us per 1000 states.  So
+// clusters serve few and large sets, more than kAlignLarge states on average for
+// each set there is: 24 sets of 65,536 states 20 us (blocks 247), 150 of them 108
+// (281), 64 of 4,096 7.9 (9.7), but 400 of 16,384 95 (80), 300 of 4,096 33 (14), 128
+// of 512 13.6 (3.1), 1000 of 256 82 (5.4).
+constexpr int kAlignCluster = 8, kAlignBlockThreads = 256;
+constexpr uint64_t kAlignLarge = 48;
+__global__ void __launch_bounds__(kAlignBlockThreads)
+    k_align_sums(const float *__restrict__ c, const float *__restrict__ den, const double2 *__restrict__ alpha,
+                 const double *__restrict__ a, const double2 *__restrict__ gamma, const double *__restrict__ E,
+                 const uint64_t *__restrict__ seg_begin, float clamp, double *__restrict__ sums) {
+    align_sums<1, kAlignBlockThreads>(blockIdx.x, 0u, c, den, alpha, a, gamma, E, seg_begin, clamp, sums);
+}
+__global__ void __launch_bounds__(kAlignThreads) __cluster_dims__(kAlignCluster, 1, 1)
+    k_align_sums_large(const float *__restrict__ c, const float *__restrict__ den, const double2 *__restrict__ alpha,
+                       const double *__restrict__ a, const double2 *__restrict__ gamma, const double *__restrict__ E,
+                       const uint64_t *__restrict__ seg_begin, float clamp, double *__restrict__ sums) {
+    align_sums<kAlignCluster, kAlignThreads>(blockIdx.x / kAlignCluster, blockIdx.x % kAlignCluster, c, den, alpha, a,
+                                             gamma, E, seg_begin, clamp, sums);
 }
 
 // dL/dc per state (zero where the clamp is active).
@@ -1442,12 +1466,15 @@ extern "C" int tcp_mlp_alignment_grad(const float *d_c, const float *d_den, cons
     if (nsets == 0) return fail(TCP_ERR_INVALID_ARGUMENT, "the alignment objective needs at least one set");
     if (!(clamp > 0.f)) return fail(TCP_ERR_INVALID_ARGUMENT, "clamp must be positive");
     cudaStream_t s = static_cast<cudaStream_t>(stream);
-    k_align_sums<<<nsets * kAlignCluster, kAlignThreads, 0, s>>>(d_c, d_den, static_cast<const double2 *>(d_alpha), d_a,
-                                                 static_cast<const double2 *>(d_gamma), d_E, d_seg_begin, clamp, d_work);
+    const auto *alpha = static_cast<const double2 *>(d_alpha), *gamma = static_cast<const double2 *>(d_gamma);
+    if (count / nsets > kAlignLarge * nsets)
+        k_align_sums_large<<<nsets * kAlignCluster, kAlignThreads, 0, s>>>(d_c, d_den, alpha, d_a, gamma, d_E,
+                                                                          d_seg_begin, clamp, d_work);
+    else
+        k_align_sums<<<nsets, kAlignBlockThreads, 0, s>>>(d_c, d_den, alpha, d_a, gamma, d_E, d_seg_begin, clamp, d_work);
     if (count > 0) {
-        k_align_dc<<<grid_for(count, 256), 256, 0, s>>>(d_c, d_den, static_cast<const double2 *>(d_alpha), d_a,
-                                                       static_cast<const double2 *>(d_gamma), d_E, d_seg, count, nsets,
-                                                       clamp, d_work, d_dc);
+        k_align_dc<<<grid_for(count, 256), 256, 0, s>>>(d_c, d_den, alpha, d_a, gamma, d_E, d_seg, count, nsets, clamp,
+                                                        d_work, d_dc);
     }
     if (d_loss) k_align_loss<<<1, 32, 0, s>>>(d_work, nsets, d_loss);
     cudaError_t e = cudaGetLastError();
