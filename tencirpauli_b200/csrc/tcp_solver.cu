@@ -446,6 +446,16 @@ __global__ void __launch_bounds__(kCombineThreads)
 // one row) serves both.  Needs n even and 16-byte aligned blocks.  n = 2^22,
 // 40 sources, 4 outputs: 338 us one row per thread, 250 two (HBM: 215).
 constexpr int kCombinePairUnroll = 8, kCombinePairBlocks = 3;  // resident blocks per SM: 80 registers
+// With more than 4 outputs a block's time is its arithmetic, and with half the row
+// blocks of one row per thread an SM that gets one more than the others shows: the
+// pairs then need 9 rounds of blocks or 93 % of the last one.  64 sources, pairs
+// against one row: 16 outputs, 460 blocks of rows 39.3 and 35.2 us, 700 blocks 45.5
+// and 47.5; 24 outputs, 600 blocks 41.3 and 37.2; 8 outputs, 1200 blocks 79.7 and
+// 88.3.  4 outputs, 600 blocks: 47.8 and 49.5.
+bool combine_by_pairs(uint32_t njp, uint64_t blocks) {
+    const uint64_t rounds = (blocks + 147) / 148;
+    return njp == 1 || rounds > 8 || 100 * blocks >= 93 * 148 * rounds;
+}
 __global__ void __launch_bounds__(kCombineThreads, kCombinePairBlocks)
     k_combine_pairs(const float4 *__restrict__ A, uint32_t p, const double2 *__restrict__ S, uint32_t k, uint32_t njp,
                     uint64_t half, double alpha, double beta, float4 *__restrict__ out) {
@@ -1334,8 +1344,9 @@ extern "C" int tcp_block_combine(const void *A, int a_dtype, uint32_t p, const v
     const bool a64 = a_dtype == TCP_DTYPE_C64, o64 = out_dtype == TCP_DTYPE_C64;
     const auto *S = static_cast<const double2 *>(d_S);
     const bool aligned = reinterpret_cast<uintptr_t>(A) % 16 == 0 && reinterpret_cast<uintptr_t>(out) % 16 == 0;
-    if (a64 && o64 && n % 2 == 0 && aligned) {
-        const int pgrid = static_cast<int>(std::min<uint64_t>((n / 2 + rb - 1) / rb, 148ull * 4 * kCombinePairBlocks));
+    const uint64_t pair_blocks = (n / 2 + rb - 1) / rb;
+    if (a64 && o64 && n % 2 == 0 && aligned && combine_by_pairs(njp, pair_blocks)) {
+        const int pgrid = static_cast<int>(std::min<uint64_t>(pair_blocks, 148ull * 4 * kCombinePairBlocks));
         cudaFuncSetAttribute(k_combine_pairs, cudaFuncAttributeMaxDynamicSharedMemorySize, 96 * 1024);
         k_combine_pairs<<<pgrid, kCombineThreads, smem, s>>>(static_cast<const float4 *>(A), p, S, k, njp, n / 2, alpha, beta,
                                                             static_cast<float4 *>(out));
