@@ -334,8 +334,14 @@ void fill_table(const AffineSpan &span, const std::vector<SignedWeight> &terms, 
 class RunTerms {
   public:
     uint64_t work = 0;  // look-ups, list steps and moves so far
+    // `zbits`: bits of the zs.  Up to 21 a bitmap of the terms left answers has()
+    // (at most 256 KiB; a bit test takes a quarter of a hash look-up).
+    explicit RunTerms(uint32_t zbits) : bitmap_(zbits <= 21) {
+        if (bitmap_) bits_.assign((size_t(1) << zbits) / 64 + 1, 0);
+    }
     // Terms of equal zs are chained behind one of them.
     void reset(const std::vector<SignedWeight> &terms) {
+        forget();
         terms_ = &terms;
         const size_t n = terms.size();
         log_ = 2;
@@ -350,10 +356,18 @@ class RunTerms {
             Slot &slot = slots_[find(terms[i].zs)];
             next_[i] = slot.at;
             slot = {terms[i].zs, i};
+            if (bitmap_) bits_[terms[i].zs >> 6] |= 1ull << (terms[i].zs & 63u);
         }
     }
-    bool has(uint32_t zs) {
+    // Clears the bitmap of the terms still left.
+    void forget() {
+        if (bitmap_ && terms_)
+            for (uint32_t i : order_) bits_[(*terms_)[i].zs >> 6] = 0;
+        terms_ = nullptr;
+    }
+    uint32_t has(uint32_t zs) {
         ++work;
+        if (bitmap_) return static_cast<uint32_t>(bits_[zs >> 6] >> (zs & 63u)) & 1u;
         return slots_[find(zs)].at < kTaken;
     }
     size_t left() const { return order_.size() - dead_; }
@@ -404,6 +418,7 @@ class RunTerms {
                 live_[i] = 0;
             }
             slot.at = kTaken;
+            if (bitmap_) bits_[zs >> 6] &= ~(1ull << (zs & 63u));
         }
         std::sort(found_.begin(), found_.end());
         dead_ += found_.size();
@@ -431,6 +446,8 @@ class RunTerms {
         return i;
     }
     const std::vector<SignedWeight> *terms_ = nullptr;
+    const bool bitmap_;
+    std::vector<uint64_t> bits_;
     uint32_t log_ = 2;
     std::vector<Slot> slots_;
     std::vector<uint32_t> next_, order_;
@@ -452,6 +469,7 @@ constexpr uint32_t kSparseTables = 64;
 // rank <= 4 become one table; larger ones are covered greedily by tables of
 // rank 4, each grown direction by direction to cover the most remaining terms.
 struct Tabulator {
+    explicit Tabulator(uint32_t zbits) : left(zbits) {}
     RunTerms left;
     std::vector<SignedWeight> in;
     std::vector<uint32_t> coords, picks, points;
@@ -504,6 +522,7 @@ struct Tabulator {
             left.tidy();
         }
         left.rest(singles);
+        left.forget();
     }
 
   private:
@@ -655,7 +674,7 @@ RingSchedule build_ring_schedule(const std::vector<MatrixTerm> &terms, uint32_t 
     };
     std::vector<SignedWeight> list, singles;
     std::vector<SignTable> tables;
-    Tabulator tabulator;
+    Tabulator tabulator(nqubits - (S - L));
     for (size_t k = 0; k < items.size();) {
         const Item first = items[k];
         if (k == 0 || first.d() != cur_d) {

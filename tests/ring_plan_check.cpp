@@ -63,8 +63,8 @@ static double diagonal(const tcp::RingSchedule &r, uint64_t row) {
 // at least 3.  Lists of up to 512 terms are rewritten after every table, longer
 // ones at 16 moves a term.  So a run takes below 64 (1000 + 512) steps and
 // (1000 + 512) / 8 more a term.
-static int work() {
-    const uint32_t n = 28;
+static int work(uint32_t n) {
+    const uint64_t mask = (1ull << n) - 1;
     auto bounded = [&](const char *name, const std::vector<MatrixTerm> &terms) {
         for (const tcp::RingShapeBits shape : tcp::kRingShapes) {
             const tcp::RingSchedule r = tcp::build_ring_schedule(terms, n, shape, shape.low == 0);
@@ -76,7 +76,7 @@ static int work() {
             // and the sum is the operator's: at most 2^18 weights of size ~1,
             // so a wrong or missing one shows; rounding alone stays below 1e-8
             for (int k = 0; k < 4 && shape.low == 0; ++k) {
-                const uint64_t row = rng() >> 36;
+                const uint64_t row = rng() & mask;
                 long double sum = 0.0L;
                 for (const MatrixTerm &t : terms) sum += odd(t.z_mask & row) ? -t.w_re : t.w_re;
                 if (std::abs(static_cast<double>(diagonal(r, row) - sum)) > 1e-8) {
@@ -88,7 +88,7 @@ static int work() {
         return true;
     };
     std::vector<MatrixTerm> t;
-    for (int k = 0; k < 1 << 18; ++k) t.push_back({0, rng() >> 36, normal(rng), 0.0});
+    for (int k = 0; k < 1 << 18; ++k) t.push_back({0, rng() & mask, normal(rng), 0.0});
     if (!bounded("random diagonal", t)) return 1;
     t.clear();
     for (uint64_t z = 0; z < 1ull << 18; ++z) t.push_back({0, z, normal(rng), 0.0});
@@ -98,7 +98,7 @@ static int work() {
     t.resize(t.size() / 4);
     if (!bounded("a quarter of it", t)) return 1;
     t.clear();
-    for (uint64_t k = 0; k < 1ull << 18; ++k) t.push_back({0, (k % 100) * 0x9e377ull & 0xfffffffull, normal(rng), 0.0});
+    for (uint64_t k = 0; k < 1ull << 18; ++k) t.push_back({0, (k % 100) * 0x9e377ull & mask, normal(rng), 0.0});
     if (!bounded("repeated words", t)) return 1;
     t.clear();
     for (uint32_t a = 0; a < n; ++a)
@@ -183,7 +183,7 @@ static int folds() {
 
 int main(int argc, char **argv) {
     const char *check = argc > 1 ? argv[1] : "";
-    if (!std::strcmp(check, "work")) return work();
+    if (!std::strcmp(check, "work")) return work(20) || work(28);  // terms left in a bitmap, in a hash table
     if (!std::strcmp(check, "folds")) return folds();
     std::printf("unknown check\n");
     return 2;
