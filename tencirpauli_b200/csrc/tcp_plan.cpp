@@ -334,9 +334,11 @@ void fill_table(const AffineSpan &span, const std::vector<SignedWeight> &terms, 
 class RunTerms {
   public:
     uint64_t work = 0;  // look-ups, list steps and moves so far
-    // `zbits`: bits of the zs.  Up to 21 a bitmap of the terms left answers has()
-    // (at most 256 KiB; a bit test takes a quarter of a hash look-up).
-    explicit RunTerms(uint32_t zbits) : bitmap_(zbits <= 21) {
+    // `zbits`: bits of the zs, `terms`: terms of the whole plan.  A bitmap of the
+    // terms left answers has() where it is small (16 KiB, or 4 bytes a term: a large
+    // one costs a small plan more to map than it saves); a bit test takes a quarter
+    // of a hash look-up.
+    RunTerms(uint32_t zbits, size_t terms) : bitmap_(((uint64_t(1) << zbits) >> 3) <= std::max<uint64_t>(16384, 4 * terms)) {
         if (bitmap_) bits_.assign((size_t(1) << zbits) / 64 + 1, 0);
     }
     // Terms of equal zs are chained behind one of them.
@@ -469,7 +471,7 @@ constexpr uint32_t kSparseTables = 64;
 // rank <= 4 become one table; larger ones are covered greedily by tables of
 // rank 4, each grown direction by direction to cover the most remaining terms.
 struct Tabulator {
-    explicit Tabulator(uint32_t zbits) : left(zbits) {}
+    Tabulator(uint32_t zbits, size_t terms) : left(zbits, terms) {}
     RunTerms left;
     std::vector<SignedWeight> in;
     std::vector<uint32_t> coords, picks, points;
@@ -674,7 +676,7 @@ RingSchedule build_ring_schedule(const std::vector<MatrixTerm> &terms, uint32_t 
     };
     std::vector<SignedWeight> list, singles;
     std::vector<SignTable> tables;
-    Tabulator tabulator(nqubits - (S - L));
+    Tabulator tabulator(nqubits - (S - L), terms.size());
     for (size_t k = 0; k < items.size();) {
         const Item first = items[k];
         if (k == 0 || first.d() != cur_d) {
