@@ -567,10 +567,11 @@ __global__ void __launch_bounds__(kU1Threads) k_u1_apply(U1Dev p, U1Apply a, siz
 // each without and with a sign mask z_out.  The value of a dead pair is not
 // loaded; complex128 adds it as 0 C, which is cheaper than a branch around it,
 // complex64 leaves it out of its compensated sum, which would turn an infinite
-// sum into NaN.  What remains is issue and the gathers from L2.  Half filling of
-// the 4 x 6 J1-J2 lattice: complex128 268 us (general kernel 376; 4 groups in
-// flight 273, 8 at 3 blocks per SM 277), complex64 258 (general kernel 369; with
-// complex products of the real constants 275).
+// sum into NaN.  What remains is the L1 data pipe (ncu: 89 % of its wavefronts, by
+// scattered gathers and table lookups).  Half filling of the 4 x 6 J1-J2 lattice:
+// complex128 268 us (general kernel 376; 4 groups in flight 273, 8 at 3 blocks per
+// SM 277), complex64 258 (general kernel 369; with complex products of the real
+// constants 275).
 // Three-level ranks (n > 24) use the "both" classes alone.
 constexpr int kU1PairBlocks = 4, kPairUnroll = 6;  // resident blocks per SM; groups in flight
 template <typename R> __device__ __forceinline__ R pair_value(uint4 r);
