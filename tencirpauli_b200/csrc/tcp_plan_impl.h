@@ -24,7 +24,7 @@ struct DeviceSchedule {
 // last piece of each direction (2^22 complex128, 64 MiB each way: 6.3 ms with
 // 4 slots of 32 MiB, 5.5 with 8 of 16, 5.06 with 16 of 8 or 32 of 4, 5.3 with 64
 // of 2; on buffers not used before 6.1 with 4 of 32, 5.1 with 16 of 8; 2^26, 1 GiB
-// each way, on another box: 61 to 67 with 4 of 32, 60 to 63 with 8 of 16, 55 to 61
+// each way, on another host: 61 to 67 with 4 of 32, 60 to 63 with 8 of 16, 55 to 61
 // with 16 of 8).
 constexpr int kStageSlots = 16;
 constexpr size_t kStageSlotBytes = size_t(8) << 20;
