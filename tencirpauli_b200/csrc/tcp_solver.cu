@@ -451,9 +451,12 @@ constexpr int kCombinePairUnroll = 8, kCombinePairBlocks = 3;  // resident block
 // pairs then need 9 rounds of blocks or 93 % of the last one.  64 sources, pairs
 // against one row: 16 outputs, 460 blocks of rows 39.3 and 35.2 us, 700 blocks 45.5
 // and 47.5; 24 outputs, 600 blocks 41.3 and 37.2; 8 outputs, 1200 blocks 79.7 and
-// 88.3.  4 outputs, 600 blocks: 47.8 and 49.5.
-bool combine_by_pairs(uint32_t njp, uint64_t blocks) {
+// 88.3.  4 outputs, 600 blocks: 47.8 and 49.5.  With 17 to 20 outputs three of a
+// block's eight tiles are padding, and the pairs gain from 13 rounds on: 20 outputs,
+// 1400 blocks 59.8 and 55.7, 2100 blocks 87.6 and 91.8.
+bool combine_by_pairs(uint32_t k, uint32_t njp, uint64_t blocks) {
     const uint64_t rounds = (blocks + 147) / 148;
+    if (k > 16 && k <= 20) return rounds > 12;
     return njp == 1 || rounds > 8 || 100 * blocks >= 93 * 148 * rounds;
 }
 __global__ void __launch_bounds__(kCombineThreads, kCombinePairBlocks)
@@ -1345,7 +1348,7 @@ extern "C" int tcp_block_combine(const void *A, int a_dtype, uint32_t p, const v
     const auto *S = static_cast<const double2 *>(d_S);
     const bool aligned = reinterpret_cast<uintptr_t>(A) % 16 == 0 && reinterpret_cast<uintptr_t>(out) % 16 == 0;
     const uint64_t pair_blocks = (n / 2 + rb - 1) / rb;
-    if (a64 && o64 && n % 2 == 0 && aligned && combine_by_pairs(njp, pair_blocks)) {
+    if (a64 && o64 && n % 2 == 0 && aligned && combine_by_pairs(k, njp, pair_blocks)) {
         const int pgrid = static_cast<int>(std::min<uint64_t>(pair_blocks, 148ull * 4 * kCombinePairBlocks));
         cudaFuncSetAttribute(k_combine_pairs, cudaFuncAttributeMaxDynamicSharedMemorySize, 96 * 1024);
         k_combine_pairs<<<pgrid, kCombineThreads, smem, s>>>(static_cast<const float4 *>(A), p, S, k, njp, n / 2, alpha, beta,

@@ -15,9 +15,9 @@ if not torch.cuda.is_available():  # pragma: no cover - CPU container
 from tencirpauli_b200 import solver_ops  # noqa: E402
 
 
-# rb rows (pairs) per block: 128 for 8 outputs, 32 for 32
-@pytest.mark.parametrize("k,rb", [(8, 128), (32, 32)])
-@pytest.mark.parametrize("blocks", [1, 137, 138, 148, 149, 275, 276, 1184, 1185])
+# rb rows (pairs) per block: 128 for 8 outputs, 32 for 20 and 32
+@pytest.mark.parametrize("k,rb", [(8, 128), (20, 32), (32, 32)])
+@pytest.mark.parametrize("blocks", [1, 137, 138, 148, 149, 275, 276, 1184, 1185, 1776, 1777])
 def test_both_kernels_give_the_same_bits(k: int, rb: int, blocks: int) -> None:
     n = 2 * rb * blocks
     gen = torch.Generator(device="cuda")
